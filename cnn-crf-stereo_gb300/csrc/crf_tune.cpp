@@ -1,7 +1,7 @@
 // crf_tune.cpp -- the CRF tile table (no counterpart in the reference, whose
 // solver has one fixed launch shape).
 //
-// A tile is the chain kernel's prefetch ring depth and chains per CTA, for
+// A tile is the chain kernel's prefetch depth (ring) and chains per CTA, for
 // the H and the V pass separately.  Which tile is fastest depends on the
 // label count D (the ring's share of shared memory), the chain lengths W and
 // H and the number of chains in flight (pairs per launch); every tile gives

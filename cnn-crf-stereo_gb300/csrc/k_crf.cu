@@ -15,7 +15,7 @@
 // Pairwise: w * rho(|t|), rho(0) = 0, rho(1..delta) per shape, L2 beyond; the
 // min-convolution is out_k = min(v_k, v_{k+-t} + w rho_t, min(v) + w L2) - min(v).
 //
-// GPU layout: one warp per chain (a row for H, a column for V); lane j holds
+// GPU layout: a warp walks each chain (a row for H, a column for V); lane j holds
 // labels k = j*P .. j*P+P-1 in registers; neighbours across lanes come from
 // warp shuffles, the minimum over labels from one redux.sync.min.f32.  All
 // operations are exact (min) or single IEEE ops in the oracle's order, so the
@@ -28,15 +28,9 @@
 namespace cnncrf {
 namespace k {
 
-int crf_pass_ring8(const CrfPassArgs &a, bool hpass, int delta, int wpb, cudaStream_t st)
+int crf_pass_p4(const CrfPassArgs &a, bool hpass, int delta, const CrfForm &f, cudaStream_t st)
 {
-    return launch_pass_any<8>(a, hpass, delta, wpb, st);
-}
-
-size_t crf_pass_smem(int P, int RING, int W, int H, bool hpass, int wpb)
-{
-    (void)W, (void)H; // the chains' weights stream through registers: no per-node shared memory
-    return sizeof(float) * wpb * (size_t)ring_floats(P, RING, hpass);
+    return launch_pass<4>(a, hpass, delta, f, st);
 }
 
 namespace {
@@ -101,21 +95,64 @@ Layout layout(int W, int H, int D, int np = 1)
     return l;
 }
 
-int pass(const CrfPassArgs &a, bool hpass, int delta, int ring, int wpb, cudaStream_t st)
-{
-    return ring == 4 ? crf_pass_ring4(a, hpass, delta, wpb, st) : crf_pass_ring8(a, hpass, delta, wpb, st);
-}
-
-// labels per lane of the instantiated kernel (launch_pass_any's choice)
+// labels per lane: ceil(D / 32) rounded up to 1, 2, 4, 6 or 8
 int lane_labels(int D)
 {
     const int P = (D + 31) / 32;
-    return P <= 4 ? P : (P <= 6 ? 6 : 8);
+    return P <= 2 ? P : (P <= 4 ? 4 : (P <= 6 ? 6 : 8));
 }
 
-bool fits(int D, int W, int H, bool hpass, int ring, int wpb)
+size_t form_smem(int D, bool hpass, bool t16, const CrfForm &f)
 {
-    return crf_pass_smem(lane_labels(D), ring, W, H, hpass, wpb) <= 227 * 1024;
+    return sizeof(float) * (f.paired ? 1 : f.wpb) * (size_t)chain_floats(lane_labels(D), hpass, t16, D % 4 != 0, f.paired, f.buffers);
+}
+
+// How a pass runs on this GPU's 152 SMs.
+//   Paired warps up to 8 chains per SM: there the sweeps' latency is the time,
+//   and the second warp takes the copies and the recomputed messages off the
+//   chain (KITTI pair, 375 row chains: 258 us paired, 316 us single).  With
+//   more chains the single warps hide each other's latency in less shared
+//   memory (1500 row chains: 604 us single, 624 us paired; 4968 column chains:
+//   481 and 526 us; 1242 column chains: 160 and 164 us), and so they do where
+//   the paired form's shared memory would not hold every chain at once.
+//   Three block buffers where that leaves every chain of the launch resident,
+//   else two (KITTI pair's row chains: 258 us with three or four, 326 us with
+//   two; 1500 row chains, single: 604 us with two, 826 us with three).  A
+//   tile's ring of 4 asks the single form for two.
+CrfForm choose_form(const CrfPassArgs &a, bool hpass, int ring, int wpb)
+{
+    constexpr long SMS = 152, SMEM_SM = 228 * 1024, SMEM_CTA = 1024; // shared memory of an SM, reserved per CTA
+    const bool t16 = hpass && a.thetaq && crf_reads_q16(a.D);
+    const long chains = (long)(hpass ? a.H : a.W) * a.np;
+    auto resident = [&](const CrfForm &f) {
+        const long ctas = (chains + (f.paired ? 1 : f.wpb) - 1) / (f.paired ? 1 : f.wpb);
+        return (long)(form_smem(a.D, hpass, t16, f) + SMEM_CTA) * ((ctas + SMS - 1) / SMS) <= SMEM_SM;
+    };
+    CrfForm f{true, 2, wpb};
+    f.paired = chains <= 8 * SMS && resident(f);
+    if (ring != 4 || f.paired) {
+        f.buffers = 3;
+        if (!resident(f)) f.buffers = 2;
+    }
+    return f;
+}
+
+int pass(const CrfPassArgs &a, bool hpass, int delta, int ring, int wpb, cudaStream_t st)
+{
+    const CrfForm f = choose_form(a, hpass, ring, wpb);
+    switch (lane_labels(a.D)) {
+    case 1: return crf_pass_p1(a, hpass, delta, f, st);
+    case 2: return crf_pass_p2(a, hpass, delta, f, st);
+    case 4: return crf_pass_p4(a, hpass, delta, f, st);
+    case 6: return crf_pass_p6(a, hpass, delta, f, st);
+    default: return crf_pass_p8(a, hpass, delta, f, st);
+    }
+}
+
+// whether a CTA of the smallest form fits (it does for every label count and wpb; an upper bound for the 16-bit unary)
+bool fits(int D, bool hpass, int wpb)
+{
+    return form_smem(D, hpass, false, CrfForm{false, 2, wpb}) <= 227 * 1024;
 }
 
 // the tile of the tuning table for this shape, each pass falling back to the
@@ -123,8 +160,8 @@ bool fits(int D, int W, int H, bool hpass, int ring, int wpb)
 CrfTile effective_tile(int W, int H, int D, int np, int delta)
 {
     CrfTile t = crf_tile_lookup(W, H, D, np, delta), d;
-    if (!fits(D, W, H, true, t.ring_h, t.wpb_h)) t.ring_h = d.ring_h, t.wpb_h = d.wpb_h;
-    if (!fits(D, W, H, false, t.ring_v, t.wpb_v)) t.ring_v = d.ring_v, t.wpb_v = d.wpb_v;
+    if (!fits(D, true, t.wpb_h)) t.ring_h = d.ring_h, t.wpb_h = d.wpb_h;
+    if (!fits(D, false, t.wpb_v)) t.ring_v = d.ring_v, t.wpb_v = d.wpb_v;
     return t;
 }
 
@@ -153,7 +190,7 @@ int run_passes(const float *cost, const float *wx, const float *wy, long wps, in
 {
     if (delta < 1 || delta > 4) return fail(CNNCRF_EUNSUPPORTED, "crf: delta %d outside 1..4", delta);
     const CrfTile t = effective_tile(W, H, D, np, delta);
-    if (!fits(D, W, H, true, t.ring_h, t.wpb_h) || !fits(D, W, H, false, t.ring_v, t.wpb_v))
+    if (!fits(D, true, t.wpb_h) || !fits(D, false, t.wpb_v))
         return fail(CNNCRF_EUNSUPPORTED, "crf: the chain ring of this tile exceeds shared memory");
     double *cH = (double *)(ws + l.ch), *cV = (double *)(ws + l.cv), *lb = (double *)(ws + l.lb);
     CrfPassArgs a = pass_args(cost, wps, W, H, D, np, rp, ws, l, costq, q);
@@ -238,7 +275,7 @@ int autotune_impl(const float *cost, const float *wx, const float *wy, long wps,
     std::vector<Cand> cands;
     for (int r : rings)
         for (int b : wpbs) {
-            Cand c{r, b, fits(D, W, H, true, r, b), fits(D, W, H, false, r, b), {}};
+            Cand c{r, b, fits(D, true, b), fits(D, false, b), {}};
             if (c.h || c.v) cands.push_back(c);
         }
     int rc = CNNCRF_OK;

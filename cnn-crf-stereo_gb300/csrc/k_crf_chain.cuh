@@ -1,8 +1,8 @@
 // k_crf_chain.cuh -- the chain pass of the CRF solve (k_crf.cu), shared by
-// the translation units that instantiate it for one prefetch depth each
-// (k_crf.cu: 8 chain steps, k_crf_r4.cu: 4), so the variants the tile tuner
-// chooses between compile in parallel.  Everything device-side has internal
-// linkage; each unit exports one launcher, crf_pass_ring<RING>.
+// the translation units that instantiate it for their label counts per lane
+// (k_crf.cu: 4, k_crf_p12.cu: 1 and 2, k_crf_p6.cu, k_crf_p8.cu), so they
+// compile in parallel.  Everything device-side has internal linkage; each
+// unit exports launchers, crf_pass_p<P>.
 #ifndef CNNCRF_K_CRF_CHAIN_CUH
 #define CNNCRF_K_CRF_CHAIN_CUH
 
@@ -40,85 +40,88 @@ struct CrfPassArgs {
     double *cmin;        // per chain minimum [np][chains]
 };
 
-// launch one pass with prefetch depth RING (4 or 8) and `wpb` warps (chains)
-// per CTA; EUNSUPPORTED when the CTA's shared memory would exceed the limit
-int crf_pass_ring8(const CrfPassArgs &a, bool hpass, int delta, int wpb, cudaStream_t st);
-int crf_pass_ring4(const CrfPassArgs &a, bool hpass, int delta, int wpb, cudaStream_t st);
-size_t crf_pass_smem(int P, int RING, int W, int H, bool hpass, int wpb);
+// how a pass runs: every choice gives the same bits
+struct CrfForm {
+    bool paired; // two warps per chain, else one
+    int buffers; // blocks of BLK nodes in shared memory (2..4)
+    int wpb;     // chains per CTA (paired: always one)
+};
+
+constexpr int BLK = 8; // chain nodes per block
+
+// launch one pass; EUNSUPPORTED when the CTA's shared memory would exceed the limit
+int crf_pass_p1(const CrfPassArgs &a, bool hpass, int delta, const CrfForm &f, cudaStream_t st);
+int crf_pass_p2(const CrfPassArgs &a, bool hpass, int delta, const CrfForm &f, cudaStream_t st);
+int crf_pass_p4(const CrfPassArgs &a, bool hpass, int delta, const CrfForm &f, cudaStream_t st);
+int crf_pass_p6(const CrfPassArgs &a, bool hpass, int delta, const CrfForm &f, cudaStream_t st);
+int crf_pass_p8(const CrfPassArgs &a, bool hpass, int delta, const CrfForm &f, cudaStream_t st);
+
+// a chain's shared memory in floats: per block buffer two planes of BLK node vectors, the unary (H pass; 16-bit codes
+// take half the floats) and phi (RAGGED vectors carry up to 3 floats of their neighbours at either end); one block of
+// messages and of edge costs, or two with paired warps
+__host__ __device__ constexpr int vec_floats(int P, bool ragged) { return 32 * P + (ragged ? 4 : 0); }
+__host__ __device__ constexpr int theta_floats(int P, bool hpass, bool t16, bool ragged)
+{
+    return hpass ? (t16 ? 16 * P : vec_floats(P, ragged)) : 0;
+}
+__host__ __device__ constexpr int block_floats(int P, bool hpass, bool t16, bool ragged)
+{
+    return BLK * (theta_floats(P, hpass, t16, ragged) + vec_floats(P, ragged));
+}
+constexpr int EDGE = 8;                // EDGE: floats of an edge's costs (w rho_1 .. w rho_4, w L2)
+constexpr int EDGES = (BLK + 1) * EDGE;       // of the edges a block uses
+__host__ __device__ constexpr int chain_floats(int P, bool hpass, bool t16, bool ragged, bool paired, int buffers)
+{
+    return buffers * block_floats(P, hpass, t16, ragged) + (paired ? 2 : 1) * (BLK * 32 * P + EDGES);
+}
 
 namespace {
 
 #define INF CUDART_INF_F
 
-// The warp minimum of the lanes' minima: one redux.sync.min.f32 (sm_100 and
-// later), exact like a float min.  The chain values are never NaN (pads are
-// +inf); a zero may come back with either sign, which no later operation
-// distinguishes (the labels compare values, the bound adds them).
-template <int P> __device__ __forceinline__ float warp_min(const float (&v)[P])
+// Exact two-lane IEEE operations (add/sub/mul/fma.rn.f32x2) and three-input
+// minimum (min.f32 with three sources): the same values as two __fadd_rn and
+// two fminf, in fewer instructions.
+__device__ __forceinline__ void add2(float a0, float a1, float b0, float b1, float &d0, float &d1)
 {
-    float m = v[0];
-#pragma unroll
-    for (int r = 1; r < P; ++r) m = fminf(m, v[r]);
-    float w;
-    asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(w) : "f"(m));
-    return w;
+    asm("{\n\t.reg .b64 ra, rb, rd;\n\t"
+        "mov.b64 ra, {%2, %3};\n\t"
+        "mov.b64 rb, {%4, %5};\n\t"
+        "add.rn.f32x2 rd, ra, rb;\n\t"
+        "mov.b64 {%0, %1}, rd;\n\t}"
+        : "=f"(d0), "=f"(d1)
+        : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
 }
-
-template <int P> __device__ __forceinline__ void load_vec(const float *p, int lane, int D, float (&v)[P])
+__device__ __forceinline__ void sub2(float a0, float a1, float b0, float b1, float &d0, float &d1)
 {
-    const int k0 = lane * P;
-    if (D == 32 * P && (P == 1 || P == 2 || P == 4 || P == 8)) {
-        if constexpr (P == 1) {
-            v[0] = p[k0];
-        } else if constexpr (P == 2) {
-            float2 t = *(const float2 *)(p + k0);
-            v[0] = t.x, v[1] = t.y;
-        } else if constexpr (P == 4) {
-            float4 t = *(const float4 *)(p + k0);
-            v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
-        } else if constexpr (P == 8) {
-            float4 t = *(const float4 *)(p + k0), u = *(const float4 *)(p + k0 + 4);
-            v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w, v[4] = u.x, v[5] = u.y, v[6] = u.z, v[7] = u.w;
-        }
-        return;
-    }
-#pragma unroll
-    for (int r = 0; r < P; ++r) v[r] = (k0 + r < D) ? p[k0 + r] : 0.0f;
+    asm("{\n\t.reg .b64 ra, rb, rd;\n\t"
+        "mov.b64 ra, {%2, %3};\n\t"
+        "mov.b64 rb, {%4, %5};\n\t"
+        "sub.rn.f32x2 rd, ra, rb;\n\t"
+        "mov.b64 {%0, %1}, rd;\n\t}"
+        : "=f"(d0), "=f"(d1)
+        : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
 }
-
-template <int P> __device__ __forceinline__ void store_vec(float *p, int lane, int D, const float (&v)[P])
-{
-    const int k0 = lane * P;
-    if (D == 32 * P && (P == 1 || P == 2 || P == 4 || P == 8)) {
-        if constexpr (P == 1) {
-            p[k0] = v[0];
-        } else if constexpr (P == 2) {
-            *(float2 *)(p + k0) = make_float2(v[0], v[1]);
-        } else if constexpr (P == 4) {
-            *(float4 *)(p + k0) = make_float4(v[0], v[1], v[2], v[3]);
-        } else if constexpr (P == 8) {
-            *(float4 *)(p + k0) = make_float4(v[0], v[1], v[2], v[3]);
-            *(float4 *)(p + k0 + 4) = make_float4(v[4], v[5], v[6], v[7]);
-        }
-        return;
-    }
-#pragma unroll
-    for (int r = 0; r < P; ++r)
-        if (k0 + r < D) p[k0 + r] = v[r];
-}
-
-// Exact two-lane IEEE add (add.rn.f32x2) and three-input minimum (min.f32
-// with three sources): the same values as two __fadd_rn and two fminf, in
-// fewer instructions.
-__device__ __forceinline__ void add2(float a0, float a1, float b, float &d0, float &d1)
+__device__ __forceinline__ void mul2(float a0, float a1, float b, float &d0, float &d1)
 {
     asm("{\n\t.reg .b64 ra, rb, rd;\n\t"
         "mov.b64 ra, {%2, %3};\n\t"
         "mov.b64 rb, {%4, %4};\n\t"
-        "add.rn.f32x2 rd, ra, rb;\n\t"
+        "mul.rn.f32x2 rd, ra, rb;\n\t"
         "mov.b64 {%0, %1}, rd;\n\t}"
         : "=f"(d0), "=f"(d1)
         : "f"(a0), "f"(a1), "f"(b));
+}
+__device__ __forceinline__ void fma2(float a0, float a1, float b, float c, float &d0, float &d1)
+{
+    asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\t"
+        "mov.b64 ra, {%2, %3};\n\t"
+        "mov.b64 rb, {%4, %4};\n\t"
+        "mov.b64 rc, {%5, %5};\n\t"
+        "fma.rn.f32x2 rd, ra, rb, rc;\n\t"
+        "mov.b64 {%0, %1}, rd;\n\t}"
+        : "=f"(d0), "=f"(d1)
+        : "f"(a0), "f"(a1), "f"(b), "f"(c));
 }
 __device__ __forceinline__ float min3(float a, float b, float c)
 {
@@ -127,126 +130,194 @@ __device__ __forceinline__ float min3(float a, float b, float c)
     return d;
 }
 
-// out = minconv(v) - g, pads (k >= D) kept at +inf.  FULL: D == 32 * P (no
-// pad labels, only the chain ends of lanes 0 and 31 are masked).
-template <int P, int DELTA, bool FULL>
-__device__ __forceinline__ void minconv(const float (&v)[P], float g, float w, const Rho &rp, int lane,
-                                        int D, float (&out)[P])
+// element-wise over a lane's P labels, in pairs
+template <int P> __device__ __forceinline__ void vadd(const float (&a)[P], const float (&b)[P], float (&d)[P])
 {
-    constexpr int NE = P + 2 * DELTA;       // labels lane*P - DELTA .. lane*P + P + DELTA - 1
-    constexpr int NE2 = (NE + 1) / 2 * 2;   // padded to whole pairs
-    float c[DELTA + 1];
 #pragma unroll
-    for (int t = 1; t <= DELTA; ++t) c[t] = __fmul_rn(w, rp.rho[t]);
-    const float base = __fadd_rn(g, __fmul_rn(w, rp.L2));
-    const int DD = FULL ? 32 * P : D;
-    // E[DELTA + i] = value at label lane*P + i, i in [-DELTA, P + DELTA)
-    float E[NE2];
+    for (int r = 0; r + 1 < P; r += 2) add2(a[r], a[r + 1], b[r], b[r + 1], d[r], d[r + 1]);
+    if constexpr (P % 2) d[P - 1] = __fadd_rn(a[P - 1], b[P - 1]);
+}
+template <int P> __device__ __forceinline__ void vsub(const float (&a)[P], const float (&b)[P], float (&d)[P])
+{
 #pragma unroll
-    for (int i = -DELTA; i < P + DELTA; ++i) {
-        float val;
-        if (i >= 0 && i < P) {
-            val = v[i];
-        } else if (i >= P) {
-            val = __shfl_down_sync(0xffffffffu, v[i % P], i / P);
-        } else {
-            int off = (-i + P - 1) / P;
-            int reg = ((i % P) + P) % P;
-            val = __shfl_up_sync(0xffffffffu, v[reg], off);
-        }
-        const int kk = lane * P + i;
-        E[DELTA + i] = (kk >= 0 && kk < DD) ? val : INF;
-    }
-    if (NE2 > NE) E[NE2 - 1] = INF;
-    float o[P];
+    for (int r = 0; r + 1 < P; r += 2) sub2(a[r], a[r + 1], b[r], b[r + 1], d[r], d[r + 1]);
+    if constexpr (P % 2) d[P - 1] = __fsub_rn(a[P - 1], b[P - 1]);
+}
+template <int P> __device__ __forceinline__ void vsub1(const float (&a)[P], float b, float (&d)[P])
+{
 #pragma unroll
-    for (int r = 0; r < P; ++r) o[r] = E[DELTA + r];
+    for (int r = 0; r + 1 < P; r += 2) sub2(a[r], a[r + 1], b, b, d[r], d[r + 1]);
+    if constexpr (P % 2) d[P - 1] = __fsub_rn(a[P - 1], b);
+}
+template <int P> __device__ __forceinline__ void vmul1(const float (&a)[P], float b, float (&d)[P])
+{
 #pragma unroll
-    for (int t = 1; t <= DELTA; ++t) {
-        float S[NE2]; // S[j] = E[j] + c[t]
-#pragma unroll
-        for (int q = 0; q < NE2; q += 2) add2(E[q], E[q + 1], c[t], S[q], S[q + 1]);
-#pragma unroll
-        for (int r = 0; r < P; ++r) o[r] = min3(o[r], S[DELTA + r - t], S[DELTA + r + t]);
-    }
-#pragma unroll
-    for (int r = 0; r < P; ++r) out[r] = (FULL || lane * P + r < D) ? __fsub_rn(fminf(o[r], base), g) : INF;
+    for (int r = 0; r + 1 < P; r += 2) mul2(a[r], a[r + 1], b, d[r], d[r + 1]);
+    if constexpr (P % 2) d[P - 1] = __fmul_rn(a[P - 1], b);
 }
 
-// ---------------------------------------------------------------- cp.async ring
+// The warp minimum of the lanes' minima: one redux.sync.min.f32 (sm_100 and
+// later), exact like a float min.  A zero may come back with either sign,
+// which no later operation distinguishes (the labels compare values, the
+// bound adds them).  The +inf operand turns a lane of pad labels, which the
+// slack hand-over leaves at NaN, into +inf.
+template <int P> __device__ __forceinline__ float warp_min(const float (&v)[P])
+{
+    float m;
+    if constexpr (P == 1) m = fminf(v[0], INF);
+    else if constexpr (P == 2) m = min3(v[0], v[1], INF);
+    else {
+        m = min3(v[0], v[1], v[2]);
+#pragma unroll
+        for (int r = 3; r + 1 < P; r += 2) m = min3(m, v[r], v[r + 1]);
+        if constexpr (P % 2 == 0) m = min3(m, v[P - 1], INF);
+    }
+    float w;
+    asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(w) : "f"(m));
+    return w;
+}
+
+// Lane constants: 0, or +inf in the lanes whose neighbour `o` lanes below
+// (lo) or above (hi) is outside the warp.  Added to a neighbour's value they
+// put +inf beyond label 0 and label 32 P - 1; labels D..32 P - 1 carry +inf
+// or NaN themselves (a minimum takes its other operand).
+template <int P, int DELTA> struct Edge {
+    static constexpr int NO = (DELTA + P - 1) / P;
+    float lo[NO + 1], hi[NO + 1];
+    __device__ __forceinline__ explicit Edge(int lane)
+    {
+#pragma unroll
+        for (int o = 1; o <= NO; ++o) lo[o] = lane < o ? INF : 0.0f, hi[o] = lane + o > 31 ? INF : 0.0f;
+    }
+};
+
+// out = minconv(v) - g with out_k = min(v_k, v_{k+-t} + w rho_t (t <= DELTA), g + w L2) - g, g = min v; cw: the edge's
+// w L2, w rho_1, ..
+template <int P, int DELTA>
+__device__ __forceinline__ void minconv(const float (&v)[P], float g, const float (&cw)[EDGE], const Edge<P, DELTA> &ed,
+                                        float (&out)[P])
+{
+    constexpr int HL = (DELTA + 1) / 2 * 2; // halo, whole pairs: E[HL + i] = value at label lane P + i
+    constexpr int NE = P + 2 * HL + (P & 1);
+    float E[NE];
+#pragma unroll
+    for (int i = 0; i < P; ++i) E[HL + i] = v[i];
+#pragma unroll
+    for (int t = 1; t <= DELTA; ++t) {
+        const int ol = (t + P - 1) / P, rl = (P - t % P) % P;          // label lane P - t
+        const int oh = (P - 1 + t) / P, rh = (P - 1 + t) % P;          // label lane P + P - 1 + t
+        E[HL - t] = __fadd_rn(__shfl_up_sync(0xffffffffu, v[rl], ol), ed.lo[ol]);
+        E[HL + P - 1 + t] = __fadd_rn(__shfl_down_sync(0xffffffffu, v[rh], oh), ed.hi[oh]);
+    }
+    float o[P];
+#pragma unroll
+    for (int r = 0; r < P; ++r) o[r] = v[r];
+#pragma unroll
+    for (int t = 1; t <= DELTA; ++t) {
+        const float c = cw[t];
+        // S[j] = E[j] + c where some label reads it: labels -t .. P-1-t and t .. P-1+t
+        float S[NE];
+        auto need = [](int i, int tt) { return (i >= -tt && i <= P - 1 - tt) || (i >= tt && i <= P - 1 + tt); };
+#pragma unroll
+        for (int i = -HL; i < P + HL; i += 2) {
+            if (need(i, t) && need(i + 1, t)) add2(E[HL + i], E[HL + i + 1], c, c, S[HL + i], S[HL + i + 1]);
+            else if (need(i, t)) S[HL + i] = __fadd_rn(E[HL + i], c);
+            else if (need(i + 1, t)) S[HL + i + 1] = __fadd_rn(E[HL + i + 1], c);
+        }
+#pragma unroll
+        for (int r = 0; r < P; ++r) o[r] = min3(o[r], S[HL + r - t], S[HL + r + t]);
+    }
+    const float base = __fadd_rn(g, cw[0]);
+#pragma unroll
+    for (int r = 0; r < P; ++r) o[r] = fminf(o[r], base);
+    vsub1<P>(o, g, out);
+}
+
+// ---------------------------------------------------------------- copies
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src)
 {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async8(uint32_t dst, const void *src)
+// the first `bytes` of a 16-byte chunk (zeros after them)
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, int bytes)
 {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void *src, int bytes)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// copy this lane's P labels of one pixel vector into its ring slot
-template <int P> __device__ __forceinline__ void lane_copy(float *dst, const float *src, int lane, int D)
+// all but the newest `left` groups (0..2) are complete
+__device__ __forceinline__ void cp_wait_left(int left)
 {
-    const int k0 = lane * P;
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst + k0);
-    if (D == 32 * P) {
-        if constexpr (P % 4 == 0) {
+    if (left == 0) cp_wait<0>();
+    else if (left == 1) cp_wait<1>();
+    else cp_wait<2>();
+}
+
+// `cnt` consecutive vectors of 32 P labels of EB bytes that lie one after the
+// other, into a plane: one flat run of 16-byte chunks
+template <int P, int EB> __device__ __forceinline__ void copy_run(uint32_t dst, const void *src, int lane, int cnt)
+{
+    constexpr int NC = BLK * 2 * P * EB; // chunks of a whole block
+    const char *g = (const char *)src + 16 * lane;
+    const uint32_t d = dst + 16 * lane;
+    if (cnt == BLK) {
 #pragma unroll
-            for (int i = 0; i < P / 4; ++i) cp_async16(d + 16 * i, src + k0 + 4 * i);
-        } else if constexpr (P % 2 == 0) {
+        for (int c = 0; c < NC; c += 32)
+            if (c + 32 <= NC || lane + c < NC) cp_async16(d + 16 * c, g + 16 * c);
+    } else {
+        for (int c = 0; lane + c < cnt * (NC / BLK); c += 32) cp_async16(d + 16 * c, g + 16 * c);
+    }
+}
+// `cnt` vectors of D labels (a multiple of 4) at a stride of ns labels, into a
+// plane.  A vector of 32 or 64 labels takes 8 or 16 lanes, so that a copy
+// instruction then carries 4 or 2 nodes.
+template <int P> __device__ __forceinline__ void copy_nodes(uint32_t dst, const float *src, long ns, int lane, int cnt, int D)
+{
+    if (P <= 2 && D == 32 * P) {
+        constexpr int LN = 8 * (P <= 2 ? P : 4), NI = 32 / LN; // lanes per node, nodes per instruction
+        const float *g = src + (lane / LN) * ns + 4 * (lane % LN);
+        const uint32_t d = dst + 16 * lane;
 #pragma unroll
-            for (int i = 0; i < P / 2; ++i) cp_async8(d + 8 * i, src + k0 + 2 * i);
+        for (int j = 0; j < BLK; j += NI, g += NI * ns)
+            if (j + lane / LN < cnt) cp_async16(d + 16 * LN * j, g);
+    } else {
+        const float *g = src + 4 * lane;
+        uint32_t d = dst + 16 * lane;
+        auto node = [&]() {
+#pragma unroll
+            for (int c = 0; c < 8 * P; c += 32)
+                if (4 * (lane + c) < D) cp_async16(d + 16 * c, g + 4 * c);
+            g += ns, d += 128 * P;
+        };
+        if (cnt == BLK) {
+#pragma unroll
+            for (int j = 0; j < BLK; ++j) node();
         } else {
-#pragma unroll
-            for (int i = 0; i < P; ++i) cp_async4(d + 4 * i, src + k0 + i, 4);
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < P; ++i) {
-            const bool ok = k0 + i < D;
-            cp_async4(d + 4 * i, ok ? src + k0 + i : src, ok ? 4 : 0);
+            for (int j = 0; j < cnt; ++j) node();
         }
     }
 }
 
-// the same for a 16-bit unary vector: this lane's P values (2P bytes, P even:
-// 4-byte aligned at any lane) into the first half of its slot
-template <int P> __device__ __forceinline__ void lane_copy16(float *dst, const uint16_t *src, int lane)
+// `cnt` vectors of any D labels from element o0 of a 16-byte aligned array of `total` elements, at a stride of ns: the
+// 16-byte chunks that hold each one (element o lands o % 4 floats into its slot), cut off at the array's end
+template <int P> __device__ __forceinline__ void copy_ragged(uint32_t dst, const float *base, long o0, long ns, long total, int lane,
+                                                             int cnt, int D)
 {
-    static_assert(P % 2 == 0, "16-bit theta copies need an even label count per lane");
-    const int k0 = lane * P;
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared((uint16_t *)dst + k0);
-    if constexpr (P % 8 == 0) {
+    uint32_t d = dst + 16 * lane;
+    long o = o0;
+    auto node = [&]() {
+        const int mis = (int)(o & 3);
+        const long c0 = o - mis + 4 * lane; // this lane's chunk
 #pragma unroll
-        for (int i = 0; i < P / 8; ++i) cp_async16(d + 16 * i, src + k0 + 8 * i);
-    } else if constexpr (P % 4 == 0) {
+        for (int c = 0; c < 8 * P + 1; c += 32)
+            if (4 * (lane + c) < D + mis) cp_async16(d + 16 * c, base + c0 + 4 * c, 4 * (int)min(4L, total - c0 - 4 * c));
+        o += ns, d += 4 * vec_floats(P, true);
+    };
+    if (cnt == BLK) {
 #pragma unroll
-        for (int i = 0; i < P / 4; ++i) cp_async8(d + 8 * i, src + k0 + 4 * i);
+        for (int j = 0; j < BLK; ++j) node();
     } else {
-#pragma unroll
-        for (int i = 0; i < P / 2; ++i) cp_async4(d + 4 * i, src + k0 + 2 * i, 4);
-    }
-}
-
-// The whole warp copies one pixel vector of NB bytes (a multiple of 16, the
-// source 16-byte aligned) into its ring slot in 16-byte chunks, lane l taking
-// chunks l, l + 32, ..: one or two copy instructions per lane, with the
-// chunk count known at compile time, where a lane copying its own labels
-// takes up to three smaller copies and a run-time check of the label count.
-// Other lanes' chunks are visible to a lane after its wait and a __syncwarp.
-template <int NB> __device__ __forceinline__ void warp_copy(void *dst, const void *src, int lane)
-{
-    static_assert(NB % 16 == 0, "whole 16-byte chunks");
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-#pragma unroll
-    for (int ch = 0; ch < (NB / 16 + 31) / 32; ++ch) {
-        const int k = lane + 32 * ch;
-        if (k < NB / 16) cp_async16(d + 16 * k, (const char *)src + 16 * k);
+        for (int j = 0; j < cnt; ++j) node();
     }
 }
 
@@ -255,305 +326,540 @@ template <int NB> __device__ __forceinline__ void warp_copy(void *dst, const voi
 // the low mantissa bits of 2^23 by one byte permute, which makes the float
 // 2^23 + q exactly, and offset23 = offset - 2^23 scale (exact, checked on the
 // host) takes the 2^23 back out inside the one rounding of the fma:
-// (2^23 + q) scale + offset23 = q scale + offset.  Two instructions per label
-// instead of a mask or shift, a conversion and the fma.
+// (2^23 + q) scale + offset23 = q scale + offset.
 template <int P>
-__device__ __forceinline__ void lane_read16(const float *slot, int lane, float scale, float offset23, float (&v)[P])
+__device__ __forceinline__ void read16(const float *slot, int lane, float scale, float offset23, float (&v)[P])
 {
-    const uint32_t *q = (const uint32_t *)((const uint16_t *)slot + lane * P);
+    uint32_t w[P / 2];
+    const uint32_t *q = (const uint32_t *)slot + lane * (P / 2);
+    if constexpr (P == 4) {
+        const uint2 t = *(const uint2 *)q;
+        w[0] = t.x, w[1] = t.y;
+    } else if constexpr (P == 8) {
+        const uint4 t = *(const uint4 *)q;
+        w[0] = t.x, w[1] = t.y, w[2] = t.z, w[3] = t.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < P / 2; ++i) w[i] = q[i];
+    }
 #pragma unroll
     for (int i = 0; i < P / 2; ++i) {
-        const uint32_t w = q[i];
-        const float lo = __int_as_float((int)__byte_perm(w, 0x4B000000u, 0x7410)); // bytes w0, w1, 0x00, 0x4B
-        const float hi = __int_as_float((int)__byte_perm(w, 0x4B000000u, 0x7432)); // bytes w2, w3, 0x00, 0x4B
-        v[2 * i] = __fmaf_rn(lo, scale, offset23);
-        v[2 * i + 1] = __fmaf_rn(hi, scale, offset23);
+        const float lo = __int_as_float((int)__byte_perm(w[i], 0x4B000000u, 0x7410)); // bytes w0, w1, 0x00, 0x4B
+        const float hi = __int_as_float((int)__byte_perm(w[i], 0x4B000000u, 0x7432)); // bytes w2, w3, 0x00, 0x4B
+        fma2(lo, hi, scale, offset23, v[2 * i], v[2 * i + 1]);
     }
 }
 
-template <int P> __device__ __forceinline__ void lane_read(const float *slot, int lane, float (&v)[P])
+// a lane's P labels of a vector in shared memory (slots are 16-byte aligned)
+template <int P> __device__ __forceinline__ void read_vec(const float *slot, int lane, float (&v)[P])
 {
-    const float *q = slot + lane * P; // 16-byte aligned for P % 4 == 0, 8-byte for P == 2
+    const float *q = slot + lane * P;
     if constexpr (P % 4 == 0) {
 #pragma unroll
-        for (int i = 0; i < P / 4; ++i) {
-            const float4 t = *(const float4 *)(q + 4 * i);
-            v[4 * i] = t.x, v[4 * i + 1] = t.y, v[4 * i + 2] = t.z, v[4 * i + 3] = t.w;
+        for (int i = 0; i < P; i += 4) {
+            const float4 t = *(const float4 *)(q + i);
+            v[i] = t.x, v[i + 1] = t.y, v[i + 2] = t.z, v[i + 3] = t.w;
         }
-    } else if constexpr (P == 2) {
-        const float2 t = *(const float2 *)q;
-        v[0] = t.x, v[1] = t.y;
+    } else if constexpr (P % 2 == 0) {
+#pragma unroll
+        for (int i = 0; i < P; i += 2) {
+            const float2 t = *(const float2 *)(q + i);
+            v[i] = t.x, v[i + 1] = t.y;
+        }
     } else {
 #pragma unroll
         for (int r = 0; r < P; ++r) v[r] = q[r];
     }
 }
 
-// floats of the ring per step: theta, phi and the forward message (H pass); phi and the message (V pass, no theta)
-// (the theta slot holds 16-bit codes when t16: half the floats)
-__host__ __device__ constexpr int theta_floats(int P, bool hpass, bool t16) { return hpass ? (t16 ? 16 * P : 32 * P) : 0; }
-__host__ __device__ constexpr int ring_floats(int P, int RING, bool hpass, bool t16 = false)
+template <int P> __device__ __forceinline__ void read_raw(const float *slot, int lane, float (&v)[P])
 {
-    return RING * (theta_floats(P, hpass, t16) + 64 * P);
+#pragma unroll
+    for (int r = 0; r < P; ++r) v[r] = slot[lane * P + r];
 }
 
-// One pass over the chains of one direction; one warp per chain.
+// store a lane's P labels to p (shared or global; the labels below D); ALIGNED: 16-byte aligned vectors, D a multiple of 4
+template <int P, bool ALIGNED> __device__ __forceinline__ void write_vec(float *p, int lane, int D, const float (&v)[P])
+{
+    const int k0 = lane * P;
+    if constexpr (ALIGNED && P % 4 == 0) {
+#pragma unroll
+        for (int i = 0; i < P; i += 4)
+            if (k0 + i < D) *(float4 *)(p + k0 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+    } else if constexpr (ALIGNED && P % 2 == 0) {
+#pragma unroll
+        for (int i = 0; i < P; i += 2)
+            if (k0 + i < D) *(float2 *)(p + k0 + i) = make_float2(v[i], v[i + 1]);
+    } else {
+#pragma unroll
+        for (int r = 0; r < P; ++r)
+            if (k0 + r < D) p[k0 + r] = v[r];
+    }
+}
+// load a lane's P labels from global memory (0 from label D on)
+template <int P, bool ALIGNED> __device__ __forceinline__ void load_vec(const float *p, int lane, int D, float (&v)[P])
+{
+    const int k0 = lane * P;
+#pragma unroll
+    for (int r = 0; r < P; ++r) v[r] = 0.0f;
+    if constexpr (ALIGNED && P % 4 == 0) {
+#pragma unroll
+        for (int i = 0; i < P; i += 4)
+            if (k0 + i < D) {
+                const float4 t = *(const float4 *)(p + k0 + i);
+                v[i] = t.x, v[i + 1] = t.y, v[i + 2] = t.z, v[i + 3] = t.w;
+            }
+    } else if constexpr (ALIGNED && P % 2 == 0) {
+#pragma unroll
+        for (int i = 0; i < P; i += 2)
+            if (k0 + i < D) {
+                const float2 t = *(const float2 *)(p + k0 + i);
+                v[i] = t.x, v[i + 1] = t.y;
+            }
+    } else {
+#pragma unroll
+        for (int r = 0; r < P; ++r)
+            if (k0 + r < D) v[r] = p[k0 + r];
+    }
+}
+
+// One pass over the chains of one direction; one or two warps per chain.
 //   HPASS: chain = row y over x (weights wx[y][x] on edge x -> x+1), unary
 //          theta - phi, the handed-over slack is added to phi.
 //   !HPASS: chain = column x over y (weights wy[y][x] on edge y -> y+1),
 //          unary phi, the handed-over slack is subtracted from phi; labels
 //          (if given) = first argmin of the min-marginals.
-// Per step the pixel vectors come from a per-warp shared-memory ring filled
-// RING steps ahead with cp.async (each lane copies and reads only its own
-// labels), so the chain's dependent arithmetic does not wait on DRAM.
-template <int P, int DELTA, bool HPASS, bool FULL, int RING, bool T16 = false, bool COOP = false>
-__global__ void __launch_bounds__(128)
-    k_crf_chain(const float *__restrict__ theta, const uint16_t *__restrict__ thetaq, float qscale, float qoffset23,
-                float *__restrict__ phi, const float *__restrict__ wgt,
-                float *__restrict__ Lbuf, int W, int H, int D, Rho rp, int first, int store_phi,
-                int32_t *__restrict__ labels, double *__restrict__ cmin_out, int npairs, long wps)
+// A chain is walked in blocks of BLK nodes.  The block's pixel vectors come
+// from a ring of block buffers in shared memory, filled `buffers` - 1 blocks
+// ahead, so that the chain's dependent arithmetic does not wait on DRAM:
+//   !RAGGED  D a multiple of 4: 16-byte cp.async by the whole warp, several
+//            nodes per instruction where they are small or contiguous
+//   RAGGED   any D: the 16-byte chunks that hold each vector
+// An edge's costs w rho_t and w L2 are multiplied out once per block, an edge
+// per lane, and read back as broadcasts.
+//
+// The forward sweep makes every node's message and the backward sweep needs
+// them again in reverse.  Only each block's first message goes to memory; the
+// others are recomputed from it, in shared memory, out of the pixel vectors
+// the backward sweep reads anyway: a third sweep of arithmetic for 2 - 2/BLK
+// fewer vectors moved per node (of the 16-bit H pass's 6 N D floats 4.25
+// remain, of the V pass's 5, 3.25).
+//   !PAIRED: one warp does it all; many chains hide its latencies.
+//   PAIRED: a second warp per chain copies the blocks in and recomputes the
+//     messages one block ahead of the first, which walks the chain: for few
+//     chains, whose time is the sweeps' latency.  The two meet at a barrier
+//     once per block; one chain per CTA.
+//
+// What bounds it: many chains, DRAM (eight KITTI pairs at D = 128: the H pass
+// 7.9 GB in 1.18 ms, 6.7 TB/s, and the V pass 6.2 GB in 0.93 ms; with all
+// messages stored and read back 1.72 and 1.38 ms).  Few chains, the latency of
+// a node's step, about 430 cycles for both sweeps of a KITTI pair's row: four
+// halo shuffles issue 4.3 cycles apart and return after 24, the warp minimum
+// after 18, and the copies of a block cost 18 cycles per instruction, which is
+// why they are few and on the second warp (one pair's H pass 470 -> 258 us,
+// its V pass 208 -> 161 us; the 256 x 192, D = 32 solve's 89 -> 40 and 70 ->
+// 34 us).  Measured and left out: bulk copies on mbarriers for the H blocks
+// (a wait costs 150 cycles, cp.async's 43; 338 against 316 us for one pair),
+// and keeping all messages for few chains (276 against 258 us).
+template <int P, int DELTA, bool HPASS, bool T16, bool RAGGED, bool PAIRED>
+__global__ void __launch_bounds__(PAIRED ? 64 : 128) k_crf_chain(const CrfPassArgs a, const int NB)
 {
     extern __shared__ float4 smem4[];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int gchain = blockIdx.x * (blockDim.x >> 5) + wib;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool walks = !PAIRED || warp == 0, helps = !PAIRED || warp == 1; // roles: walk the chain; copy and recompute
+    const int wib = PAIRED ? 0 : warp; // the chain within the CTA
+    const int gchain = PAIRED ? blockIdx.x : blockIdx.x * (blockDim.x >> 5) + wib;
+    const int W = a.W, H = a.H, D = T16 ? 32 * P : a.D;
     const int n = HPASS ? W : H;
     const int nch = HPASS ? H : W;
-    if (gchain >= nch * npairs) return;
+    if (gchain >= nch * a.np) return;
     // pair of the batch and chain within it
     const int pair = gchain / nch, chain = gchain - pair * nch;
-    const long pnd = (long)W * H * D * pair;
-    theta += pnd;
-    if (T16) thetaq += pnd;
-    phi += pnd;
-    Lbuf += pnd;
-    wgt += wps * pair;
-    if (labels) labels += (long)W * H * pair;
-    cmin_out += (long)nch * pair;
-    float *ring = (float *)smem4 + (size_t)wib * ring_floats(P, RING, HPASS, T16);
-    auto pix = [&](int i) -> long { return HPASS ? (long)chain * W + i : (long)i * W + chain; };
-    // Edge weights in registers: lane l holds the weight of edge 32 b + l of
-    // the sweep's current block b (wc) and of the block it reaches next (wn),
-    // one load per lane and block; a step's weight is a shuffle that depends
-    // on no chain state, so shared memory does not grow with the chain.
-    auto wload = [&](int b) -> float {
-        const int e = 32 * b + lane;
-        return (b >= 0 && e < n) ? __ldg(wgt + pix(e)) : 0.0f;
-    };
-    const bool use_phi = !(HPASS && first);
-    // slot a of step i: 0 theta (H pass only), 1 phi, 2 the forward message
-    constexpr int TF = theta_floats(P, HPASS, T16), SF = TF + 64 * P;
-    auto slot = [&](int i, int a) { return ring + (i % RING) * SF + (a == 0 ? 0 : TF + (a - 1) * 32 * P); };
+    // element offset of the chain's node 0 and the stride between its nodes
+    const long ns = (HPASS ? 1L : (long)W) * D;
+    const long cb = (long)W * H * D * pair + (HPASS ? (long)chain * W : (long)chain) * D;
+    const float *theta = a.theta + cb;
+    const uint16_t *thetaq = T16 ? a.thetaq + cb : nullptr;
+    float *phi = a.phi + cb;
+    float *lbuf = a.lbuf + cb;
+    const float *wgt = a.wgt + a.wps * pair + (HPASS ? (long)chain * W : (long)chain);
+    const long wst = HPASS ? 1 : W; // weight of edge e (node e to e + 1) at wgt[e wst]
 
-    // element offsets of the chain's nodes: node i at cb + i ns; the sweeps
-    // step running offsets by ns instead of multiplying per node
-    const long cb = pix(0) * D, ns = (HPASS ? 1L : (long)W) * D;
+    constexpr bool RAG = RAGGED, VEC = !RAG; // VEC: 16-byte aligned vectors of a multiple of 4 labels
+    constexpr int LP = 32 * P, VF = vec_floats(P, RAG), TF = theta_floats(P, HPASS, T16, RAG);
+    constexpr int OP = BLK * TF; // planes of a buffer: the unary at 0, phi at OP
+    constexpr int BF = block_floats(P, HPASS, T16, RAG), MF = BLK * LP + EDGES;
+    float *ring = (float *)smem4 + (size_t)wib * chain_floats(P, HPASS, T16, RAG, PAIRED, NB);
+    float *msg = ring + NB * BF; // the block's messages and edge costs (PAIRED: of even and odd blocks of the sweep)
+    const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring);
+    const bool use_phi = !(HPASS && a.first);
 
-    // ---- forward: messages into each node, stored for the backward sweep
-    // COOP (label counts that fill whole warps, 16-byte aligned vectors): the
-    // warp copies each vector in 16-byte chunks instead of each lane its labels
-    static_assert(!COOP || FULL, "cooperative copies: label counts that fill whole warps");
-    auto issue_f = [&](int i, long o) { // node i, at element offset o
-        if (i < n) {
-            if constexpr (COOP) {
-                if constexpr (HPASS && T16) warp_copy<64 * P>(slot(i, 0), thetaq + o, lane);
-                else if (HPASS) warp_copy<128 * P>(slot(i, 0), theta + o, lane);
-                if (use_phi) warp_copy<128 * P>(slot(i, 1), phi + o, lane);
-            } else {
-                if constexpr (HPASS && T16) lane_copy16<P>(slot(i, 0), thetaq + o, lane);
-                else if (HPASS) lane_copy<P>(slot(i, 0), theta + o, lane, D);
-                if (use_phi) lane_copy<P>(slot(i, 1), phi + o, lane, D);
+    // Labels D..32 P - 1 are pads at +inf: set once, the copies never write
+    // them (RAGGED slots hold other vectors' labels there, and read_node masks
+    // them).  The first H pass copies no phi: zero.
+    if (helps && (D < LP || !use_phi)) {
+        for (int i = lane; i < NB * BLK * VF; i += 32) {
+            const int nd = i / VF, k = i - nd * VF, q = nd / BLK, j = nd - q * BLK;
+            float *s = ring + q * BF;
+            const bool pad = k >= D;
+            if (HPASS) {
+                if (!T16 && pad) s[j * TF + k] = INF;
+                if (pad || !use_phi) s[OP + j * VF + k] = 0.0f;
+            } else if (pad) {
+                s[OP + j * VF + k] = INF;
             }
+        }
+    }
+    __syncwarp();
+
+    const int nblk = (n + BLK - 1) / BLK;
+    int ibuf = 0; // the buffer of the next copied block
+    // copy block b into the next buffer
+    auto issue = [&](int b) {
+        if (b >= 0 && b < nblk) {
+            const int i0 = b * BLK, cnt = min(BLK, n - i0);
+            const uint32_t d = ring_s + (uint32_t)(ibuf * BF) * 4u;
+            const long o = (long)i0 * ns;
+            if constexpr (!RAG) {
+                if (HPASS && D == LP) {
+                    if constexpr (T16) copy_run<P, 2>(d, thetaq + o, lane, cnt);
+                    else copy_run<P, 4>(d, theta + o, lane, cnt);
+                    if (use_phi) copy_run<P, 4>(d + OP * 4, phi + o, lane, cnt);
+                } else {
+                    if (HPASS) copy_nodes<P>(d, theta + o, ns, lane, cnt, D);
+                    if (use_phi) copy_nodes<P>(d + OP * 4, phi + o, ns, lane, cnt, D);
+                }
+            } else {
+                const long total = (long)W * H * D * a.np;
+                if (HPASS) copy_ragged<P>(d, a.theta, cb + o, ns, total, lane, cnt, D);
+                if (use_phi) copy_ragged<P>(d + OP * 4, a.phi, cb + o, ns, total, lane, cnt, D);
+            }
+            ibuf = ibuf + 1 == NB ? 0 : ibuf + 1;
         }
         cp_commit();
     };
-    float L[P], v[P], th[P], ph[P];
-#pragma unroll
-    for (int r = 0; r < P; ++r) L[r] = 0.0f, th[r] = 0.0f, ph[r] = 0.0f;
-    long po = cb, so = cb; // the node being prefetched, the node being stored
-    for (int i = 0; i < RING - 1; ++i, po += ns) issue_f(i, po);
-    // the chain's minimum in FP64: lane l sums the node minima g_i of i = l mod 32
-    // in ascending i, and the 32 partial sums are added in lane order at the end
-    // of the sweep.  Within a block of 32 nodes lane l keeps node 32 b + l's
-    // minimum as a float (gb) and adds it once, at the block's end: one FP64
-    // conversion and add per 32 nodes, none on the message chain
-    double acc = 0.0;
-    float wn = wload(0);
-    // blocks of 32 nodes: the block's weights in wc, the next block's loading into wn
-    for (int b = 0, i = 0; i < n; ++b) {
-    const float wc = wn;
-    wn = wload(b + 1);
-    const int iend = min(n, i + 32), nb = iend - i;
-    float gb = 0.0f;
-#pragma unroll (HPASS ? 1 : 2)
-    for (; i < iend; ++i) {
-        issue_f(i + RING - 1, po);
-        po += ns;
-        cp_wait<RING - 1>();
-        if constexpr (COOP) __syncwarp(); // the other lanes' chunks of node i
-        if constexpr (HPASS && T16) lane_read16<P>(slot(i, 0), lane, qscale, qoffset23, th);
-        else if (HPASS) lane_read<P>(slot(i, 0), lane, th);
-        if (use_phi) lane_read<P>(slot(i, 1), lane, ph);
-        store_vec<P>(Lbuf + so, lane, D, L);
-        so += ns;
-#pragma unroll
-        for (int r = 0; r < P; ++r) {
-            const float un = HPASS ? __fsub_rn(th[r], ph[r]) : ph[r];
-            v[r] = (FULL || lane * P + r < D) ? __fadd_rn(L[r], un) : INF;
-        }
-        const float g = warp_min<P>(v);
-        gb = lane == (i & 31) ? g : gb;
-        if (i < n - 1) minconv<P, DELTA, FULL>(v, g, __shfl_sync(0xffffffffu, wc, i & 31), rp, lane, D, L);
-    }
-    if (lane < nb) acc += (double)gb;
-    }
-    cp_wait<0>();
-    double cmin = acc; // lane 0: ((p0 + p1) + p2) + ... + p31
-#pragma unroll 1
-    for (int l = 1; l < 32; ++l) {
-        const double pl = __shfl_sync(0xffffffffu, acc, l);
-        if (lane == 0) cmin += pl;
-    }
-
-    // ---- backward: min-marginals, slack hand-over, reduced unary propagated back
-    auto issue_b = [&](int j, long o) { // j-th step of the sweep = node n-1-j, at element offset o
-        if (j < n) {
-            if constexpr (COOP) {
-                if constexpr (HPASS && T16) warp_copy<64 * P>(slot(j, 0), thetaq + o, lane);
-                else if (HPASS) warp_copy<128 * P>(slot(j, 0), theta + o, lane);
-                if (use_phi) warp_copy<128 * P>(slot(j, 1), phi + o, lane);
-                warp_copy<128 * P>(slot(j, 2), Lbuf + o, lane);
-            } else {
-                if constexpr (HPASS && T16) lane_copy16<P>(slot(j, 0), thetaq + o, lane);
-                else if (HPASS) lane_copy<P>(slot(j, 0), theta + o, lane, D);
-                if (use_phi) lane_copy<P>(slot(j, 1), phi + o, lane, D);
-                lane_copy<P>(slot(j, 2), Lbuf + o, lane, D);
-            }
-        }
-        cp_commit();
+    // the next block is in its buffer, every lane is done with the one before it
+    int buf = 0;
+    auto arrived = [&]() {
+        cp_wait_left(NB - 2);
+        __syncwarp();
     };
-    float R[P], Lx[P], m[P], A[P];
+    // PAIRED: the two warps of the chain (the CTA) meet
+    auto meet = [&]() {
+        if constexpr (PAIRED) __syncthreads();
+    };
+    auto next_buf = [&]() -> const float * {
+        const float *p = ring + buf * BF;
+        buf = buf + 1 == NB ? 0 : buf + 1;
+        return p;
+    };
+    // lane l < BLK + 1: the weight of edge BLK b - 1 + l
+    auto weights = [&](int b) -> float {
+        const int e = b * BLK - 1 + lane;
+        return (b >= 0 && lane <= BLK && e >= 0 && e < n - 1) ? __ldg(wgt + (long)e * wst) : 0.0f;
+    };
+    // that edge's costs: w L2, w rho_1, .., w rho_DELTA
+    auto edge_costs = [&](float w, float *ec) {
+        float c[EDGE];
+        c[0] = __fmul_rn(w, a.rp.L2);
 #pragma unroll
-    for (int r = 0; r < P; ++r) R[r] = 0.0f;
-    po = so = cb + (long)(n - 1) * ns;                 // both sweep down from node n-1
-    long lpix = pix(n - 1);                            // the label's pixel (V pass)
-    for (int j = 0; j < RING - 1; ++j, po -= ns) issue_b(j, po);
-    // the sweep reads edges n-2 down to 0, in blocks of 32 edges from the top;
-    // node 0 (no edge below it) comes last, in a block of its own
-    wn = wload((n - 2) >> 5);
-    for (int eb = (n - 2) >> 5, j = 0; j < n; --eb) {
-    const float wc = wn;
-    wn = wload(eb - 1);
-    const int jend = eb >= 0 ? n - 1 - 32 * eb : n; // nodes i = e + 1 for the block's edges e
-#pragma unroll (HPASS ? 1 : 2)
-    for (; j < jend; ++j) {
-        const int i = n - 1 - j, e = i - 1; // edge e -> i
-        issue_b(j + RING - 1, po);
-        po -= ns;
-        cp_wait<RING - 1>();
-        if constexpr (COOP) __syncwarp();
-        if constexpr (HPASS && T16) lane_read16<P>(slot(j, 0), lane, qscale, qoffset23, th);
-        else if (HPASS) lane_read<P>(slot(j, 0), lane, th);
-        if (use_phi) {
-            lane_read<P>(slot(j, 1), lane, ph);
+        for (int t = 1; t < EDGE; ++t) c[t] = t <= DELTA ? __fmul_rn(w, a.rp.rho[t]) : 0.0f;
+        if (lane <= BLK) {
+            *(float4 *)(ec + lane * EDGE) = make_float4(c[0], c[1], c[2], c[3]);
+            if (DELTA > 3) ec[lane * EDGE + 4] = c[4];
+        }
+    };
+    // a node's inputs: the subproblem's unary (theta - phi, or phi), phi, and the costs of the edge its message crosses.
+    // Every sweep reads them one node ahead of the chain's arithmetic, which so waits neither on shared memory nor on
+    // the dequantisation
+    struct Node {
+        float un[P], ph[P], vm[P], cw[EDGE];
+    };
+    auto read_plane = [&](const float *bs, int j, long o, float (&x)[P]) {
+        if constexpr (RAG) read_raw<P>(bs + j * VF + (int)(o & 3), lane, x);
+        else read_vec<P>(bs + j * VF, lane, x);
+    };
+    auto read_node = [&](const float *bs, int i0, int j, Node &nd) {
+        const long o = RAG ? cb + (long)(i0 + j) * ns : 0;
+        if constexpr (HPASS) {
+            float th[P];
+            if constexpr (T16) read16<P>(bs + j * TF, lane, a.qscale, a.qoffset23, th);
+            else read_plane(bs, j, o, th);
+            read_plane(bs + OP, j, o, nd.ph);
+            vsub<P>(th, nd.ph, nd.un);
         } else {
-#pragma unroll
-            for (int r = 0; r < P; ++r) ph[r] = 0.0f; // phi starts at zero
+            read_plane(bs + OP, j, o, nd.un);
         }
-        lane_read<P>(slot(j, 2), lane, Lx);
+        if constexpr (RAG)
 #pragma unroll
-        for (int r = 0; r < P; ++r) {
-            A[r] = HPASS ? __fsub_rn(th[r], ph[r]) : ph[r];
-            m[r] = (FULL || lane * P + r < D) ? __fadd_rn(__fadd_rn(Lx[r], A[r]), R[r]) : INF;
+            for (int r = 0; r < P; ++r) nd.un[r] = lane * P + r < D ? nd.un[r] : INF;
+    };
+    auto read_edge = [&](const float *ec, int j, Node &nd) { // slot j: edge i0 - 1 + j
+        const float4 t = *(const float4 *)(ec + j * EDGE);
+        nd.cw[0] = t.x, nd.cw[1] = t.y, nd.cw[2] = t.z, nd.cw[3] = t.w;
+        if (DELTA > 3) nd.cw[4] = ec[j * EDGE + 4];
+    };
+
+    const Edge<P, DELTA> ed(lane);
+    float L[P], v[P];
+    Node cur, nxt;
+#pragma unroll
+    for (int r = 0; r < P; ++r) L[r] = 0.0f;
+
+    double cmin = 0.0;
+    float R[P], m[P], Lc[P];
+#pragma unroll
+    for (int r = 0; r < P; ++r) R[r] = 0.0f, Lc[r] = 0.0f;
+
+    // block b again from its first message, Lc: message plus unary of every node, into ms; the first message of the
+    // sweep's next block loads meanwhile
+    auto recompute = [&](int b, const float *bs, float *ms) {
+        const int i0 = b * BLK, cnt = min(BLK, n - i0);
+        const float *ec = ms + BLK * LP;
+#pragma unroll
+        for (int r = 0; r < P; ++r) L[r] = b > 0 ? Lc[r] : 0.0f;
+        if (b > 1) load_vec<P, VEC>(lbuf + (long)(b - 1) * BLK * ns, lane, D, Lc);
+        read_node(bs, i0, 0, nxt);
+        read_edge(ec, 1, nxt);
+        auto again = [&](int j, bool more) { // more: another node follows in the block
+            cur = nxt;
+            if (more) {
+                read_node(bs, i0, j + 1, nxt);
+                read_edge(ec, j + 2, nxt);
+            }
+            vadd<P>(L, cur.un, v);
+            write_vec<P, true>(ms + j * LP, lane, LP, v);
+            if (more) {
+                const float g = warp_min<P>(v);
+                minconv<P, DELTA>(v, g, cur.cw, ed, L);
+            }
+        };
+        if (cnt == BLK) {
+#pragma unroll
+            for (int j = 0; j < BLK; ++j) again(j, j < BLK - 1);
+        } else {
+#pragma unroll 1
+            for (int j = 0; j < cnt; ++j) again(j, j < cnt - 1);
         }
-        const float mu = warp_min<P>(m);
-        if (!HPASS && labels) {
-            int best = 0x7fffffff;
-#pragma unroll
-            for (int r = P - 1; r >= 0; --r)
-                if (m[r] == mu && (FULL || lane * P + r < D)) best = lane * P + r;
-            best = __reduce_min_sync(0xffffffffu, best);
-            if (lane == 0) labels[lpix] = best;
-            lpix -= W;
+    };
+
+    if (PAIRED && !walks) { // ---- the second warp: copies, and the messages of the backward sweep
+        float wn = weights(0), *ms = msg;
+        for (int b = 0; b < NB - 1; ++b) issue(b);
+        for (int b = 0; b < nblk; ++b) {
+            edge_costs(wn, ms + BLK * LP);
+            wn = weights(b + 1);
+            ms = ms == msg ? msg + MF : msg;
+            arrived();
+            meet(); // block b is there; block b - 1's buffer is free
+            issue(b + NB - 1);
+            next_buf();
         }
-#pragma unroll
-        for (int r = 0; r < P; ++r) {
-            const float h = __fmul_rn(rp.slack, __fsub_rn(m[r], mu));
-            A[r] = __fsub_rn(A[r], h);
-            ph[r] = HPASS ? __fadd_rn(ph[r], h) : A[r];
+        cp_wait<0>();
+        meet(); // the first messages are in memory
+        for (int q = 0; q < NB - 1; ++q) issue(nblk - 1 - q);
+        if (nblk > 1) load_vec<P, VEC>(lbuf + (long)(nblk - 1) * BLK * ns, lane, D, Lc);
+        wn = weights(nblk - 1), ms = msg;
+        for (int b = nblk - 1; b >= 0; --b) {
+            edge_costs(wn, ms + BLK * LP);
+            wn = weights(b - 1);
+            arrived();
+            recompute(b, next_buf(), ms);
+            meet(); // block b and its messages are there; block b + 1's buffers are free
+            issue(b - (NB - 1));
+            ms = ms == msg ? msg + MF : msg;
         }
-        if (store_phi) store_vec<P>(phi + so, lane, D, ph);
-        so -= ns;
-        if (i > 0) {
-#pragma unroll
-            for (int r = 0; r < P; ++r) v[r] = (FULL || lane * P + r < D) ? __fadd_rn(A[r], R[r]) : INF;
+        cp_wait<0>();
+        return;
+    }
+
+    // ---- forward: messages into each node.  The chain's minimum in FP64:
+    // lane l sums the node minima g_i of i = l mod 32 in ascending i, and the
+    // 32 partial sums are added in lane order at the end of the sweep.  Lane l
+    // keeps node 32 b + l's minimum as a float (gb) and adds it once per 32
+    // nodes: no FP64 operation on the message chain
+    double acc = 0.0;
+    float gb = 0.0f;
+    if (!PAIRED)
+        for (int b = 0; b < NB - 1; ++b) issue(b);
+    float wn = PAIRED ? 0.0f : weights(0), *ms = msg;
+    long so = 0; // element offset of the node being stored
+    for (int b = 0; b < nblk; ++b) {
+        meet();
+        if (!PAIRED) {
+            arrived();
+            issue(b + NB - 1);
+        }
+        const float *bs = next_buf(), *ec = ms + BLK * LP;
+        if (PAIRED) {
+            ms = ms == msg ? msg + MF : msg;
+        } else {
+            edge_costs(wn, ms + BLK * LP);
+            wn = weights(b + 1);
+            __syncwarp();
+        }
+        const int i0 = b * BLK, cnt = min(BLK, n - i0), gl = lane - (i0 & 31);
+        if (b > 0) write_vec<P, VEC>(lbuf + so, lane, D, L);
+        so += BLK * ns;
+        read_node(bs, i0, 0, nxt);
+        read_edge(ec, 1, nxt);
+        auto step = [&](int j, bool more, bool last) { // more: node j + 1 is in the block
+            cur = nxt;
+            if (more) {
+                read_node(bs, i0, j + 1, nxt);
+                read_edge(ec, j + 2, nxt);
+            }
+            vadd<P>(L, cur.un, v);
             const float g = warp_min<P>(v);
-            minconv<P, DELTA, FULL>(v, g, __shfl_sync(0xffffffffu, wc, e & 31), rp, lane, D, R);
+            gb = gl == j ? g : gb;
+            if (!last) minconv<P, DELTA>(v, g, cur.cw, ed, L);
+        };
+        if (b < nblk - 1) {
+#pragma unroll
+            for (int j = 0; j < BLK; ++j) step(j, j < BLK - 1, false);
+        } else {
+#pragma unroll 1
+            for (int j = 0; j < cnt; ++j) step(j, j < cnt - 1, j == cnt - 1);
+        }
+        if (b == nblk - 1 || (i0 & 31) == 32 - BLK) {
+            if (lane < (i0 & 31) + cnt) acc += (double)gb;
         }
     }
+    if (!PAIRED) cp_wait<0>();
+
+    // ---- backward: min-marginals, slack hand-over, reduced unary propagated back.
+    // The chain minimum ((p0 + p1) + p2) + ... + p31 is added up meanwhile, two
+    // partial sums per block: 31 dependent FP64 adds take about 3100 cycles
+    cmin = __shfl_sync(0xffffffffu, acc, 0);
+    int part = 1;
+    auto add_part = [&]() {
+        if (part < 32) cmin += __shfl_sync(0xffffffffu, acc, part);
+        ++part;
+    };
+    __syncwarp();
+    meet();
+    const int Dst = a.store_phi ? D : 0; // labels of phi to store
+    if (!PAIRED) {
+        for (int q = 0; q < NB - 1; ++q) issue(nblk - 1 - q);
+        if (nblk > 1) load_vec<P, VEC>(lbuf + (long)(nblk - 1) * BLK * ns, lane, D, Lc);
+        wn = weights(nblk - 1);
     }
-    cp_wait<0>();
-    if (lane == 0) cmin_out[chain] = cmin;
+    ms = msg;
+    for (int b = nblk - 1; b >= 0; --b) {
+        meet();
+        if (!PAIRED) {
+            arrived();
+            issue(b - (NB - 1));
+        }
+        const float *bs = next_buf(), *ec = ms + BLK * LP;
+        const int i0 = b * BLK, cnt = min(BLK, n - i0);
+        add_part();
+        add_part();
+        if (!PAIRED) {
+            edge_costs(wn, ms + BLK * LP);
+            wn = weights(b - 1);
+            __syncwarp();
+            recompute(b, bs, ms);
+        }
+        auto read_back = [&](int j) {
+            read_node(bs, i0, j, nxt);
+            read_vec<P>(ms + j * LP, lane, nxt.vm);
+            read_edge(ec, j, nxt);
+        };
+        read_back(cnt - 1);
+        auto back = [&](int j, bool first, bool want) { // first: node 0 of the chain; want: labels
+            cur = nxt;
+            if (j > 0) read_back(j - 1);
+            vadd<P>(cur.vm, R, m);
+            const float mu = warp_min<P>(m);
+            if (!HPASS && want) {
+                int best = 0x7fffffff;
+#pragma unroll
+                for (int r = P - 1; r >= 0; --r)
+                    if (m[r] == mu) best = lane * P + r;
+                best = __reduce_min_sync(0xffffffffu, best);
+                if (lane == 0) a.labels[(long)W * H * pair + (long)(i0 + j) * W + chain] = best;
+            }
+            float h[P], A[P];
+            vsub1<P>(m, mu, h);
+            vmul1<P>(h, a.rp.slack, h);
+            vsub<P>(cur.un, h, A);
+            if constexpr (HPASS) vadd<P>(cur.ph, h, cur.ph);
+            write_vec<P, VEC>(phi + so, lane, Dst, HPASS ? cur.ph : A);
+            so -= ns;
+            if (!first) {
+                vadd<P>(A, R, v);
+                const float g = warp_min<P>(v);
+                minconv<P, DELTA>(v, g, cur.cw, ed, R);
+            }
+        };
+        so = (long)(i0 + cnt - 1) * ns;
+        if (cnt == BLK && b > 0 && !a.labels) {
+#pragma unroll
+            for (int j = BLK - 1; j >= 0; --j) back(j, false, false);
+        } else {
+            const bool want = a.labels != nullptr;
+#pragma unroll 1
+            for (int j = cnt - 1; j >= 0; --j) back(j, i0 + j == 0, want);
+        }
+        if (PAIRED) ms = ms == msg ? msg + MF : msg;
+    }
+    if (!PAIRED) cp_wait<0>();
+    while (part < 32) add_part();
+    if (lane == 0) a.cmin[(long)nch * pair + chain] = cmin;
 }
 
-template <int P, int DELTA, int RING>
-int launch_pass(const CrfPassArgs &a, bool hpass, int wpb, cudaStream_t st)
+template <int P, int DELTA, bool HPASS, bool T16, bool RAGGED, bool PAIRED>
+int launch_form_as(const CrfPassArgs &a, const CrfForm &f, cudaStream_t st)
 {
-    const bool full = a.D == 32 * P;
-    // the H pass on the 16-bit unary where each lane's labels are an even count (aligned copies)
-    const bool t16 = hpass && full && a.thetaq != nullptr && P % 2 == 0;
-    const size_t sm = sizeof(float) * wpb * (size_t)ring_floats(P, RING, hpass, t16);
+    const int wpb = PAIRED ? 1 : f.wpb;
+    const size_t sm = sizeof(float) * wpb * (size_t)chain_floats(P, HPASS, T16, RAGGED, PAIRED, f.buffers);
     if (sm > 227 * 1024) return fail(CNNCRF_EUNSUPPORTED, "crf: %zu bytes of ring per CTA", sm);
-    auto kern = hpass ? (full ? k_crf_chain<P, DELTA, true, true, RING> : k_crf_chain<P, DELTA, true, false, RING>)
-                      : (full ? k_crf_chain<P, DELTA, false, true, RING> : k_crf_chain<P, DELTA, false, false, RING>);
-    if constexpr (P % 2 == 0)
-        if (t16) kern = k_crf_chain<P, DELTA, true, true, RING, true>;
-    // cooperative 16-byte copies where the vectors allow them (the workspace's phi and messages are 256-byte
-    // aligned; a caller's cost volume may not be)
-    {
-        const bool aligned = (((uintptr_t)a.theta | (uintptr_t)a.thetaq | (uintptr_t)a.phi | (uintptr_t)a.lbuf) & 15) == 0;
-        if (full && aligned) {
-            if (!hpass) kern = k_crf_chain<P, DELTA, false, true, RING, false, true>;
-            else if (t16) kern = k_crf_chain<P, DELTA, true, true, RING, P % 2 == 0, true>;
-            else kern = k_crf_chain<P, DELTA, true, true, RING, false, true>;
-        }
-    }
+    auto kern = k_crf_chain<P, DELTA, HPASS, T16, RAGGED, PAIRED>;
     CNNCRF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    const long chains = (long)(hpass ? a.H : a.W) * a.np;
+    const long chains = (long)(HPASS ? a.H : a.W) * a.np;
     {
-        CNNCRF_PROF(hpass ? "crf_h" : "crf_v", st);
-        kern<<<ceil_div(chains, wpb), 32 * wpb, sm, st>>>(a.theta, a.thetaq, a.qscale, a.qoffset23, a.phi, a.wgt,
-                                                           a.lbuf, a.W, a.H, a.D, a.rp,
-                                                           a.first, a.store_phi, a.labels, a.cmin, a.np,
-                                                           a.wps);
+        CNNCRF_PROF(HPASS ? "crf_h" : "crf_v", st);
+        kern<<<ceil_div(chains, wpb), (PAIRED ? 64 : 32) * wpb, sm, st>>>(a, f.buffers);
     }
     CNNCRF_CHECK_LAUNCH();
     return CNNCRF_OK;
 }
 
-template <int P, int RING>
-int launch_pass_delta(const CrfPassArgs &a, bool hpass, int delta, int wpb, cudaStream_t st)
+template <int P, int DELTA, bool HPASS, bool T16>
+int launch_form(const CrfPassArgs &a, const CrfForm &f, cudaStream_t st)
 {
-    switch (delta) {
-    case 1: return launch_pass<P, 1, RING>(a, hpass, wpb, st);
-    case 2: return launch_pass<P, 2, RING>(a, hpass, wpb, st);
-    case 3: return launch_pass<P, 3, RING>(a, hpass, wpb, st);
-    case 4: return launch_pass<P, 4, RING>(a, hpass, wpb, st);
-    default: return fail(CNNCRF_EUNSUPPORTED, "crf: delta %d outside 1..4", delta);
-    }
+    // whole 16-byte chunks where the vectors allow them (the solver's arrays start on 16 bytes: the workspace's by its
+    // layout, a caller's cost volume by check_args)
+    if (a.D % 4 == 0)
+        return f.paired ? launch_form_as<P, DELTA, HPASS, T16, false, true>(a, f, st)
+                        : launch_form_as<P, DELTA, HPASS, T16, false, false>(a, f, st);
+    if constexpr (T16) return fail(CNNCRF_EINVAL, "crf: 16-bit unary at depth %d", a.D); // crf_reads_q16: never
+    else
+        return f.paired ? launch_form_as<P, DELTA, HPASS, T16, true, true>(a, f, st)
+                        : launch_form_as<P, DELTA, HPASS, T16, true, false>(a, f, st);
 }
 
-// labels per lane P = ceil(D / 32) rounded up to 1, 2, 3, 4, 6 or 8
-template <int RING>
-int launch_pass_any(const CrfPassArgs &a, bool hpass, int delta, int wpb, cudaStream_t st)
+template <int P, int DELTA> int launch_dir(const CrfPassArgs &a, bool hpass, const CrfForm &f, cudaStream_t st)
 {
-    if (wpb < 1 || wpb > 4) return fail(CNNCRF_EINVAL, "crf: %d chains per CTA outside 1..4", wpb);
-    const int P = (a.D + 31) / 32;
-    if (P <= 1) return launch_pass_delta<1, RING>(a, hpass, delta, wpb, st);
-    if (P <= 2) return launch_pass_delta<2, RING>(a, hpass, delta, wpb, st);
-    if (P <= 3) return launch_pass_delta<3, RING>(a, hpass, delta, wpb, st);
-    if (P <= 4) return launch_pass_delta<4, RING>(a, hpass, delta, wpb, st);
-    if (P <= 6) return launch_pass_delta<6, RING>(a, hpass, delta, wpb, st);
-    return launch_pass_delta<8, RING>(a, hpass, delta, wpb, st);
+    if (!hpass) return launch_form<P, DELTA, false, false>(a, f, st);
+    // the H pass on the 16-bit unary where the labels fill the lanes with an even count (aligned copies)
+    if constexpr (P % 2 == 0)
+        if (a.thetaq && a.D == 32 * P) return launch_form<P, DELTA, true, true>(a, f, st);
+    return launch_form<P, DELTA, true, false>(a, f, st);
+}
+
+template <int P> int launch_pass(const CrfPassArgs &a, bool hpass, int delta, const CrfForm &f, cudaStream_t st)
+{
+    if (f.wpb < 1 || f.wpb > 4) return fail(CNNCRF_EINVAL, "crf: %d chains per CTA outside 1..4", f.wpb);
+    if (f.buffers < 2 || f.buffers > 4) return fail(CNNCRF_EINVAL, "crf: %d block buffers outside 2..4", f.buffers);
+    if (delta < 1 || delta > 4) return fail(CNNCRF_EUNSUPPORTED, "crf: delta %d outside 1..4", delta);
+    switch (delta) {
+    case 1: return launch_dir<P, 1>(a, hpass, f, st);
+    case 2: return launch_dir<P, 2>(a, hpass, f, st);
+    case 3: return launch_dir<P, 3>(a, hpass, f, st);
+    default: return launch_dir<P, 4>(a, hpass, f, st);
+    }
 }
 
 } // namespace

@@ -252,8 +252,9 @@ void slackprop_set_costq(struct ::cnncrf_slackprop *sp, const void *costq, Unary
 int crf_c1(const float *cost, const void *ws, long n, float *out, cudaStream_t st, int D = 0,
            const void *costq = nullptr, UnaryQ16 q = UnaryQ16{0.0f, 0.0f});
 
-// CRF tile: prefetch ring depth (4 or 8 chain steps) and chains (warps) per
-// CTA (1, 2 or 4) of the H and the V pass.  Every tile gives the same bits;
+// CRF tile: prefetch depth (4: two blocks of nodes, 8: three where shared memory
+// holds every chain so) and chains per CTA (1, 2 or 4; a pass with few chains
+// always runs one) of the H and the V pass.  Every tile gives the same bits;
 // only the speed differs.  The solver takes the tile of the process-wide
 // tuning table for (W, H, D, npairs, delta), the default if there is none.
 struct CrfTile {

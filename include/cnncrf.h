@@ -259,9 +259,11 @@ int cnncrf_crf_solve_static(const float *d_cost, const float *d_wx, const float 
                             double *lower_bound, cnncrf_stream_t stream);
 
 /* CRF tiles.  No counterpart in the reference, whose solver has one launch
- * shape.  A tile is the chain kernel's prefetch ring depth (4 or 8 chain
- * steps) and chains per CTA (1, 2 or 4) for the horizontal and the vertical
- * pass.  Every tile gives the same labels and bound bit for bit; the fastest
+ * shape.  A tile is the chain kernel's prefetch depth (ring 8: three blocks of
+ * 8 nodes where shared memory then holds every chain of the launch, else two;
+ * ring 4: two) and chains per CTA (1, 2 or 4) for the horizontal and the
+ * vertical pass; passes with few chains (up to 8 per SM) run two warps per
+ * chain, one chain per CTA, and three blocks at either depth.  Every tile gives the same labels and bound bit for bit; the fastest
  * depends on the label count, the chain lengths and the pairs per launch, so
  * the library keeps a process-wide table from (width, height, depth, npairs,
  * delta) to a tile.  Every solve (cnncrf_crf_solve, SlackProp, Stereo, the
