@@ -853,7 +853,11 @@ template <int P> int launch_pass(const CrfPassArgs &a, bool hpass, int delta, co
 {
     if (f.wpb < 1 || f.wpb > 4) return fail(CNNCRF_EINVAL, "crf: %d chains per CTA outside 1..4", f.wpb);
     if (f.buffers < 2 || f.buffers > 4) return fail(CNNCRF_EINVAL, "crf: %d block buffers outside 2..4", f.buffers);
+    // An offset whose rho reaches L2 never wins over the truncation: v_{k+-t} >= g, and adding the same w L2 rounds
+    // monotonically, so v_{k+-t} + w rho_t >= g + w L2.  Those offsets are left out (the repository's truncated linear
+    // term, L1 = 0.5, L2 = 1.5 at delta 3, computes two of its three), with the same bits
     if (delta < 1 || delta > 4) return fail(CNNCRF_EUNSUPPORTED, "crf: delta %d outside 1..4", delta);
+    while (delta > 1 && a.rp.rho[delta] >= a.rp.L2) --delta;
     switch (delta) {
     case 1: return launch_dir<P, 1>(a, hpass, f, st);
     case 2: return launch_dir<P, 2>(a, hpass, f, st);

@@ -2,8 +2,8 @@
 buffers, whole 16-byte vectors or ragged ones) at the sizes where they can go
 wrong, against the oracle bit for bit: chain lengths around the 8-node blocks
 and the 32-node sums, label counts around the lanes' 1, 2, 4, 6 and 8 labels
-and off the 4-label chunks, and chain counts on both sides of the paired
-form's limit."""
+and off the 4-label chunks, chain counts on both sides of the paired form's
+limit, and the offsets that the truncation makes redundant."""
 import numpy as np
 import pytest
 
@@ -42,3 +42,9 @@ def test_label_counts(cuda, oracle, D, delta):
 def test_chain_counts(cuda, oracle, H, W, D):
     check(cuda, oracle, H, W, D, 0.5, 1.5, 3, 1)
 
+
+@pytest.mark.parametrize("L1,L2,delta,shape", [(0.5, 1.5, 3, 1), (0.5, 1.5, 4, 1), (2.0, 1.0, 4, 1), (3.0, 2.0, 3, 0), (0.5, 1.51, 3, 1)])
+@pytest.mark.parametrize("D", [30, 96])
+def test_redundant_offsets(cuda, oracle, L1, L2, delta, shape, D):
+    """rho at the far offsets reaches L2 (or just does not): the kernels leave them out (or not)."""
+    check(cuda, oracle, 17, 21, D, L1, L2, delta, shape, iters=3)
