@@ -7,8 +7,12 @@
 // CUDNN_CONVOLUTION mode + cudnnAddTensor + tanh, stereo/operators/
 // convolution.cpp:141-152, bias.cpp:58-67, activation.cpp:33-41).
 //
-// Tiling: CTA = 128 pixels of one output row x 128 output channels, k-slices
-// of 8 double-buffered in shared memory, 256 threads with 8x8 register tiles.
+// k_conv_px and k_conv_patch carry the nets' layers; k_conv_nt and k_conv_simt
+// (CTA = 128 pixels of one output row x up to 128 output channels, k-slices
+// double-buffered in shared memory, 8x8 register tiles) the other shapes.
+#include <algorithm>
+#include <type_traits>
+
 #include <cuda_bf16.h>
 
 #include "../../include/cnncrf_fmath.h"
@@ -145,7 +149,8 @@ __device__ __forceinline__ void fma2(unsigned long long &acc, unsigned long long
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
 
-// The same convolution with the channel tile cut to the layer's width (TN =
+// The layers that k_conv_px does not take (thin or oddly aligned inputs, up to
+// 32 or over 104 channels, BF16 outputs).  The same convolution with the channel tile cut to the layer's width (TN =
 // 32, 64 or 112 output channels, for Cout <= TN) and the index arithmetic
 // taken out of the k loop.  2 TN threads, each an 8 x 8 register tile (8
 // pixels x 8 channels); k-slices of TK (7 at TN = 112, else 8), so that every
@@ -293,68 +298,253 @@ __global__ void __launch_bounds__(2 * TN, 2) k_conv_nt(ConvArgs a, int Ho, int W
     }
 }
 
-// First layers (Cin <= 5): one thread per output pixel holds all COUT
-// accumulators; its 3x3xCin patch sits in registers and the weights are read
-// from shared memory as broadcast float4.  Same per-output order as above:
-// k = (ky, kx, ci) ascending, one fmaf per term, then + bias, activation.
-template <int COUT>
-__global__ void __launch_bounds__(128) k_conv_first(ConvArgs a, int Ho, int Wo, int K)
+// The wide layers (Cin a multiple of 16 or 20, 16-byte aligned pixels): a CTA
+// of four warps computes 128 output pixels, taken in row order across row
+// ends so that narrow images leave no part of a tile idle; lane l has pixels
+// l, l + 32, l + 64, l + 96 of it, warp w channels CPW w .. CPW w + CPW - 1.
+// Four k steps of a warp are four 16-byte loads of its pixels' inputs
+// (conflict-free at a pitch of 20 floats), broadcast loads of its weights and
+// 8 CPW packed fmas; every scheduler carries the same two warps.  k-slices of
+// TK, which divides Cin: a slice lies inside one tap and its input offset is
+// the same for every pixel.  Inputs and weights come by cp.async, PXS slices
+// deep.  Per output the terms in ascending k, one fmaf each: the same bits as
+// k_conv_nt.
+//
+// Bound by the FMA pipe: fma.rn.f32x2 issues every 2.5 cycles (measured alone
+// 2.48 to 2.7), 130 cycles per warp and k step at CPW = 26; the 3x3 layers of
+// a 720 x 480 pair take about 155 with the epilogue.  All FP32 convolutions of
+// that pair with its re-match: 33.4 -> 24.9 ms; of a KITTI pair in 2x2 layers
+// 14.5 -> 11.5 ms; of a 256 x 192 grey pair 4.58 -> 2.93 ms (k_conv_nt: 14
+// warps per SM on four schedulers, 8 pack moves per 32 fmas, a row's last
+// tile).  Measured and left out: three CTAs at 168 registers (spills, 26.0
+// ms), scalar fmas (33.3 ms), exactly 25 channels per warp with one unpaired
+// (25.3 ms).
+constexpr int PXT = 128, PXS = 3, PXP = 20; // pixels per CTA, slices in flight, floats of a pixel's slice
+__host__ __device__ constexpr int cpw_pitch(int CPW) { return (CPW + 3) / 4 * 4; } // floats of a warp's weights per k
+__host__ __device__ constexpr int epi_pitch(int CPW) { return CPW / 2 % 2 ? CPW : CPW + 2; } // floats of a pixel in the epilogue
+__host__ __device__ constexpr int px_stage(int CPW, int TK) { return PXT * PXP + TK * 4 * cpw_pitch(CPW); }
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src)
 {
-    constexpr int CP = (COUT + 3) & ~3;
-    extern __shared__ float4 wsm4[];
-    float *wsm = (float *)wsm4; // [K][CP]
-    for (int i = threadIdx.x; i < K * CP; i += blockDim.x) {
-        int k = i / CP, co = i - k * CP;
-        wsm[i] = a.wt[(long)k * BN + co];
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// accumulators of 4 pixels x CPW / 2 channel pairs; four (or kn) k steps on them: A the lane's pixel, B the warp's weights
+template <int CPW> struct PxAcc {
+    unsigned long long v[4][CPW / 2];
+    __device__ __forceinline__ PxAcc()
+    {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int m = 0; m < CPW / 2; ++m) v[i][m] = 0ull;
     }
-    __syncthreads();
-    const int oy = blockIdx.y, ox = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ox >= Wo) return;
-    a.in += (long)blockIdx.z * a.in_img; // image of the batch
-    if (a.out16) a.out16 = (char *)a.out16 + (long)blockIdx.z * a.out_img * 2;
-    else a.out += (long)blockIdx.z * a.out_img;
-    // channel pairs (2m, 2m+1), one packed fma per pair and term
-    unsigned long long acc2[CP / 2];
+    // ap: the pixels' input of this k, duplicated
+    __device__ __forceinline__ void step(const unsigned long long (&ap)[4], const float *b)
+    {
 #pragma unroll
-    for (int m = 0; m < CP / 2; ++m) acc2[m] = 0ull;
-    for (int ky = 0; ky < a.kh; ++ky)
-        for (int kx = 0; kx < a.kw; ++kx) {
-            const float *src = a.in + (long)(oy + ky) * a.in_row + (long)(ox + kx) * a.in_pix;
-            const int kb = (ky * a.kw + kx) * a.Cin;
-            for (int ci = 0; ci < a.Cin; ++ci) {
-                const float xv = __ldg(src + ci);
-                const unsigned long long xp = pack2(xv, xv);
-                const ulonglong2 *w = (const ulonglong2 *)(wsm + (kb + ci) * CP);
+        for (int m = 0; m + 1 < CPW / 2; m += 2) {
+            const ulonglong2 bv = *(const ulonglong2 *)(b + 2 * m);
 #pragma unroll
-                for (int q = 0; q < CP / 4; ++q) {
-                    const ulonglong2 wv = w[q];
-                    fma2(acc2[2 * q], xp, wv.x);
-                    fma2(acc2[2 * q + 1], xp, wv.y);
-                }
+            for (int i = 0; i < 4; ++i) fma2(v[i][m], ap[i], bv.x), fma2(v[i][m + 1], ap[i], bv.y);
+        }
+        if (CPW / 2 % 2) {
+            const unsigned long long bv = *(const unsigned long long *)(b + CPW - 2);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) fma2(v[i][CPW / 2 - 1], ap[i], bv);
+        }
+    }
+    template <int PITCH> __device__ __forceinline__ void steps(const float *A, const float *B, int kn = 4)
+    {
+        constexpr int WB = 4 * cpw_pitch(CPW);
+        float av[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 t = *(const float4 *)(A + 32 * PITCH * i);
+            av[i][0] = t.x, av[i][1] = t.y, av[i][2] = t.z, av[i][3] = t.w;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (k >= kn) break;
+            unsigned long long ap[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) ap[i] = pack2(av[i][k], av[i][k]);
+            step(ap, B + k * WB);
+        }
+    }
+};
+
+// The warp's 128 pixels x CPW channels through shared memory, then a rolled loop of bias, activation and store on
+// channel pairs, a pixel's channels as one run (unrolled on the registers, the activations were 66 KB of code that
+// every CTA ran through once).  The pitch makes a column of pairs conflict-free
+template <int CPW>
+__device__ __forceinline__ void px_epilogue(const ConvArgs &a, const PxAcc<CPW> &acc, float *sm, float *outp, int p0, int npx,
+                                            int Wo, int lane, int warp)
+{
+    constexpr int EP = epi_pitch(CPW);
+    float *st = sm + warp * PXT * EP;
+    const int c0 = warp * CPW, nc = min(CPW, a.Cout - c0);
+    if (nc <= 0) return;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int m = 0; m < CPW / 2; ++m) *(unsigned long long *)(st + (lane + 32 * i) * EP + 2 * m) = acc.v[i][m];
+    __syncwarp();
+    const bool dense = a.out_ch == 1 && a.out_row == Wo * a.out_pix;
+    const bool pairs = dense && a.out_pix % 2 == 0 && nc % 2 == 0 && ((uintptr_t)outp & 7) == 0;
+    const int np = (nc + 1) / 2, dq = 32 / np, dm = 32 - dq * np; // channel pairs; a lane's stride in pixels and pairs
+    int q = lane / np, m = lane - q * np;
+#pragma unroll 1
+    for (int e = lane; e < PXT * np; e += 32) {
+        const int c = 2 * m, p = p0 + q;
+        if (p < npx) {
+            float2 t = *(const float2 *)(st + q * EP + c);
+            if (a.bias) t.x = __fadd_rn(t.x, __ldg(a.bias + c0 + c)), t.y = __fadd_rn(t.y, __ldg(a.bias + c0 + c + 1));
+            t.x = act_fn(t.x, a.act), t.y = act_fn(t.y, a.act);
+            if (pairs) {
+                *(float2 *)(outp + (long)p * a.out_pix + c0 + c) = t;
+            } else {
+                const int y = dense ? 0 : p / Wo, x = p - y * Wo;
+                float *o = outp + (long)y * a.out_row + (long)x * a.out_pix + (long)(c0 + c) * a.out_ch;
+                o[0] = t.x;
+                if (c + 1 < nc) o[a.out_ch] = t.y;
             }
         }
-    float acc[CP];
-#pragma unroll
-    for (int m = 0; m < CP / 2; ++m) asm("mov.b64 {%0, %1}, %2;" : "=f"(acc[2 * m]), "=f"(acc[2 * m + 1]) : "l"(acc2[m]));
-#pragma unroll
-    for (int co = 0; co < CP; ++co) {
-        float v = acc[co];
-        if (a.bias) v = __fadd_rn(v, a.bias[co]);
-        acc[co] = act_fn(v, a.act);
+        m += dm, q += dq;
+        if (m >= np) m -= np, ++q;
     }
-    const long pix = (long)oy * Wo + ox;
-    if (a.out16) {
-        __nv_bfloat16 *d16 = (__nv_bfloat16 *)a.out16 + pix * a.out_cs;
+}
+
+template <int CPW, int TK>
+__global__ void __launch_bounds__(128, 2) k_conv_px(ConvArgs a, int npx, int Wo, int K)
+{
+    constexpr int NQ = TK / 4;         // 16-byte pieces of a pixel's slice
+    constexpr int PP = cpw_pitch(CPW); // a warp's weights per k
+    constexpr int WB = 4 * PP;         // a k row of weights
+    constexpr int SF = px_stage(CPW, TK);
+    static_assert(CPW % 2 == 0 && TK % 4 == 0 && TK <= PXP && 4 * CPW <= BN, "k_conv_px tile");
+    extern __shared__ float4 sm4[];
+    float *sm = (float *)sm4; // [PXS][PXT][PXP] inputs and [TK][WB] weights
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int p0 = blockIdx.x * PXT;
+    const float *in = a.in + (long)blockIdx.y * a.in_img; // image of the batch
+    float *outp = a.out + (long)blockIdx.y * a.out_img;
+    // loader: piece q of a pixel, 128 NQ pieces over 128 threads, the piece fastest; its input offset without the
+    // slice's, and its place in a stage
+    int poff[NQ];
+    uint32_t pdst[NQ];
+    const uint32_t sm_s = (uint32_t)__cvta_generic_to_shared(sm);
 #pragma unroll
-        for (int co = 0; co < COUT; co += 2) {
-            const float v1 = co + 1 < COUT ? acc[co + 1] : 0.0f;
-            *(__nv_bfloat162 *)(d16 + co) = __floats2bfloat162_rn(acc[co], v1);
+    for (int j = 0; j < NQ; ++j) {
+        const int f = tid + 128 * j, px = f / NQ, q = f - px * NQ;
+        const int p = min(p0 + px, npx - 1), y = p / Wo, x = p - y * Wo; // the last tile's idle pixels repeat the last one
+        poff[j] = y * (int)a.in_row + x * (int)a.in_pix + 4 * q;
+        pdst[j] = sm_s + 4 * (px * PXP + 4 * q);
+    }
+    const int nsl = K / TK;
+    // the slice being loaded: tap column kx, first channel ci
+    int kx = 0, ci = 0, ls = 0, lbuf = 0;
+    const float *src = in, *wsrc = a.wt;
+    auto load = [&]() {
+        if (ls < nsl) {
+            const uint32_t o = 4u * SF * lbuf;
+#pragma unroll
+            for (int j = 0; j < NQ; ++j) cp_async16(pdst[j] + o, src + poff[j]);
+            constexpr int CF = CPW % 4 == 0 ? 4 : 2, NC = CPW / CF; // floats of a copy, copies per warp and k
+            const uint32_t d = sm_s + o + 4 * PXT * PXP;
+#pragma unroll
+            for (int f0 = 0; f0 < TK * 4 * NC; f0 += 128) {
+                const int f = f0 + tid;
+                if (f < TK * 4 * NC) {
+                    const int k = f / (4 * NC), r = f - k * (4 * NC), g = r / NC, c = r - g * NC;
+                    const uint32_t dst = d + (k * WB + g * PP + c * CF) * 4;
+                    if (CF == 4) cp_async16(dst, wsrc + k * BN + g * CPW + c * CF);
+                    else cp_async8(dst, wsrc + k * BN + g * CPW + c * CF);
+                }
+            }
+            wsrc += TK * BN;
+            ci += TK, src += TK;
+            if (ci == a.Cin) {
+                ci = 0, src += a.in_pix - a.Cin;
+                if (++kx == a.kw) kx = 0, src += a.in_row - a.kw * a.in_pix;
+            }
+            ++ls, lbuf = lbuf + 1 == PXS ? 0 : lbuf + 1;
         }
-    } else {
-        float *d = a.out + pix * a.Cout;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    PxAcc<CPW> acc;
+    for (int s = 0; s < PXS - 1; ++s) load();
+    for (int s = 0, cur = 0; s < nsl; ++s, cur = cur + 1 == PXS ? 0 : cur + 1) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(PXS - 2) : "memory");
+        __syncthreads(); // slice s is there; everyone is done with slice s - 1
+        load();
+        const float *A = sm + cur * SF + lane * PXP, *B = sm + cur * SF + PXT * PXP + warp * PP;
 #pragma unroll
-        for (int co = 0; co < COUT; ++co) d[co] = acc[co];
+        for (int q = 0; q < NQ; ++q, A += 4, B += 4 * WB) acc.template steps<PXP>(A, B);
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    px_epilogue<CPW>(a, acc, sm, outp, p0, npx, Wo, lane, warp);
+}
+
+// First layers (thin inputs): the same tile, with the 128 pixels' patches of K
+// = kh kw Cin <= KP values gathered whole, [pixel][KP] at a conflict-free
+// pitch, and all K rows of the weights in shared memory.  Bound by the tanh
+// epilogue and the output's bytes; a thread per pixel with all channels in
+// registers stored 4 bytes at a 400-byte stride and took 1.42 ms for a KITTI
+// pair's three first layers, this 0.76.
+template <int CPW, int KP>
+__global__ void __launch_bounds__(128, 3) k_conv_patch(ConvArgs a, int npx, int Wo, int K)
+{
+    constexpr int PP = cpw_pitch(CPW), WB = 4 * PP;
+    static_assert(KP % 8 == 4, "conflict-free pixel pitch");
+    extern __shared__ float4 sm4[];
+    float *A = (float *)sm4, *B = A + PXT * KP; // [PXT][KP], [K][WB]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int p0 = blockIdx.x * PXT;
+    float *outp = a.out + (long)blockIdx.y * a.out_img;
+    {
+        const int p = min(p0 + tid, npx - 1), y = p / Wo, x = p - y * Wo; // this thread's pixel (idle ones repeat the last)
+        const float *src = a.in + (long)blockIdx.y * a.in_img + (long)y * a.in_row + (long)x * a.in_pix;
+        float *d = A + tid * KP;
+        for (int ky = 0; ky < a.kh; ++ky)
+            for (int kx = 0; kx < a.kw; ++kx)
+                for (int ci = 0; ci < a.Cin; ++ci) *d++ = __ldg(src + (long)ky * a.in_row + (long)kx * a.in_pix + ci);
+    }
+    for (int i = tid; i < K * 4 * CPW; i += 128) {
+        const int k = i / (4 * CPW), c = i - k * (4 * CPW), g = c / CPW;
+        B[k * WB + g * PP + c - g * CPW] = __ldg(a.wt + (long)k * BN + c);
+    }
+    __syncthreads();
+    PxAcc<CPW> acc;
+    const float *Ap = A + lane * KP, *Bp = B + warp * PP;
+#pragma unroll 1
+    for (int k = 0; k < K; k += 4, Ap += 4, Bp += 4 * WB) acc.template steps<KP>(Ap, Bp, K - k);
+    __syncthreads();
+    px_epilogue<CPW>(a, acc, A, outp, p0, npx, Wo, lane, warp);
+}
+
+template <int CPW, int TK> int launch_px(const ConvArgs &a, int Ho, int Wo, int K, cudaStream_t st)
+{
+    const int sm = 4 * std::max(PXS * px_stage(CPW, TK), 4 * PXT * epi_pitch(CPW));
+    CNNCRF_CUDA(cudaFuncSetAttribute(k_conv_px<CPW, TK>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+    CNNCRF_PROF("conv_simt", st);
+    k_conv_px<CPW, TK><<<dim3(ceil_div((long)Ho * Wo, PXT), a.n_img), 128, sm, st>>>(a, Ho * Wo, Wo, K);
+    return CNNCRF_OK;
+}
+
+template <int CPW, int KP> int launch_patch(const ConvArgs &a, int Ho, int Wo, int K, cudaStream_t st)
+{
+    const int sm = 4 * std::max(PXT * KP + K * 4 * cpw_pitch(CPW), 4 * PXT * epi_pitch(CPW));
+    CNNCRF_CUDA(cudaFuncSetAttribute(k_conv_patch<CPW, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+    CNNCRF_PROF("conv_first", st);
+    k_conv_patch<CPW, KP><<<dim3(ceil_div((long)Ho * Wo, PXT), a.n_img), 128, sm, st>>>(a, Ho * Wo, Wo, K);
+    return CNNCRF_OK;
 }
 
 __global__ void k_head2(const float *__restrict__ in, int npx, int Cin, const float *__restrict__ w,
@@ -417,18 +607,34 @@ int conv_simt(const ConvArgs &args, cudaStream_t st)
     int K = a.kh * a.kw * a.Cin;
     const bool dense = a.out_pix == 0;
     if (dense) a.out_pix = a.Cout, a.out_row = (long)Wo * a.Cout, a.out_ch = 1;
-    if (dense && K <= 45 && (a.Cout == 100 || a.Cout == 64) && a.Cout == (a.Cout & ~1)) {
-        dim3 g(ceil_div(Wo, 128), Ho, a.n_img);
-        size_t smem = sizeof(float) * (size_t)K * ((a.Cout + 3) & ~3);
-        if (a.Cout == 100) {
-            CNNCRF_PROF("conv_first", st);
-            k_conv_first<100><<<g, 128, smem, st>>>(a, Ho, Wo, K);
-        } else {
-            CNNCRF_PROF("conv_first", st);
-            k_conv_first<64><<<g, 128, smem, st>>>(a, Ho, Wo, K);
-        }
+    // k_conv_patch: K = 9 (grey), 27 (RGB), 45 (RGB and coordinates) of a first 3x3 layer
+    if (!a.out16 && K <= 52 && a.Cout > 32 && a.Cout <= 104 && (long)Ho * Wo < (1L << 31) && a.n_img <= 65535) {
+        auto launch = [&](auto cpw) {
+            constexpr int CPW = decltype(cpw)::value;
+            return K <= 12   ? launch_patch<CPW, 12>(a, Ho, Wo, K, st)
+                   : K <= 28 ? launch_patch<CPW, 28>(a, Ho, Wo, K, st)
+                             : launch_patch<CPW, 52>(a, Ho, Wo, K, st);
+        };
+        CNNCRF_TRY(a.Cout <= 64 ? launch(std::integral_constant<int, 16>()) : launch(std::integral_constant<int, 26>()));
         CNNCRF_CHECK_LAUNCH();
         return CNNCRF_OK;
+    }
+    // k_conv_px: 16-byte pixels, slices inside a tap, 32-bit offsets within an image
+    const bool al16 = (((uintptr_t)a.in | (uintptr_t)a.wt) & 15) == 0 && a.in_pix % 4 == 0 && a.in_row % 4 == 0 &&
+                      a.in_img % 4 == 0 && a.Cin % 4 == 0;
+    const bool off32 = (long)a.H * a.in_row < (1L << 31) && (long)Ho * Wo < (1L << 31);
+    if (al16 && off32 && !a.out16 && a.n_img <= 65535 && (a.Cin % 20 == 0 || a.Cin % 16 == 0)) {
+        const bool t20 = a.Cin % 20 == 0;
+        if (a.Cout > 64 && a.Cout <= 104) {
+            CNNCRF_TRY((t20 ? launch_px<26, 20>(a, Ho, Wo, K, st) : launch_px<26, 16>(a, Ho, Wo, K, st)));
+            CNNCRF_CHECK_LAUNCH();
+            return CNNCRF_OK;
+        }
+        if (a.Cout > 32 && a.Cout <= 64) {
+            CNNCRF_TRY((t20 ? launch_px<16, 20>(a, Ho, Wo, K, st) : launch_px<16, 16>(a, Ho, Wo, K, st)));
+            CNNCRF_CHECK_LAUNCH();
+            return CNNCRF_OK;
+        }
     }
     dim3 grid(ceil_div(Wo, BM), Ho, a.n_img);
     {
