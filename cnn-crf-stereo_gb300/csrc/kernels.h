@@ -205,9 +205,9 @@ int train_sgd(float *theta, const float *g, float *v, long n, float lr, float mu
 constexpr int GAUSS_R = 3;           // Gaussian of the edge image: radius 3 >= 3 sigma
 constexpr float GAUSS_SIGMA = 0.7f;  // stereo/stereo.cu:1092
 int rgb_to_gray(const float *rgba, long n, float *gray, cudaStream_t st);
-// d_list[z] = the z-th disparity (positive = left pixel x matches right x - d)
-int census_volume(const float *g1, const float *g2, int W, int H, int fs, const float *d_list, int D, float lambda,
-                  float *vol, cudaStream_t st);
+// d_list[z] = h_list[z] = the z-th disparity (positive = left pixel x matches right x - d)
+int census_volume(const float *g1, const float *g2, int W, int H, int fs, const float *d_list, const float *h_list, int D,
+                  float lambda, float *vol, cudaStream_t st);
 void gauss_weights(float sigma, int R, float *w); // host: 2R+1 normalised weights
 int edge_weights(const float *gray, int W, int H, float alpha, float beta, float lambda, float *tmp, float *tmp2,
                  const float *d_gw, float *wx, float *wy, cudaStream_t st);

@@ -319,7 +319,7 @@ int cnncrf_census_volume(const float *d_gray_ref, const float *d_gray_other, int
     DevBuf dl;
     CNNCRF_TRY(dl.reserve(sizeof(float) * depth));
     CNNCRF_CUDA(cudaMemcpyAsync(dl.get(), l.data(), sizeof(float) * depth, cudaMemcpyHostToDevice, st));
-    CNNCRF_TRY(k::census_volume(d_gray_ref, d_gray_other, width, height, filter_size, dl.as<float>(), depth, lambda,
+    CNNCRF_TRY(k::census_volume(d_gray_ref, d_gray_other, width, height, filter_size, dl.as<float>(), l.data(), depth, lambda,
                                 d_volume, st));
     CNNCRF_CUDA(cudaStreamSynchronize(st)); // the list buffer is freed on return
     return CNNCRF_OK;

@@ -122,8 +122,8 @@ int cnncrf_stereo::census(int lr)
     for (int z = 0; z < depth; ++z, d += dstep) dlist_host[z] = d;
     CNNCRF_CUDA(cudaMemcpyAsync(dlist.get(), dlist_host.data(), sizeof(float) * depth, cudaMemcpyHostToDevice, st));
     const int a = lr ? 0 : 1;
-    return k::census_volume(gray[a].as<float>(), gray[1 - a].as<float>(), W, H, filter_size, dlist.as<float>(), depth,
-                            1.0f, vol.as<float>(), st);
+    return k::census_volume(gray[a].as<float>(), gray[1 - a].as<float>(), W, H, filter_size, dlist.as<float>(),
+                            dlist_host.data(), depth, 1.0f, vol.as<float>(), st);
 }
 
 // computeWeights: calcEdgeImage of the reference side's grey image
