@@ -380,5 +380,11 @@ int crf_c1(const float *cost, const void *ws, long n, float *out, cudaStream_t s
     return CNNCRF_OK;
 }
 
+int crf_quadfit(float *u, const float *cost, const void *ws, long npx, int D, float dmin, float dstep, cudaStream_t st,
+                const void *costq, UnaryQ16 q)
+{
+    return quadfit_solver(u, cost, costq && crf_reads_q16(D) ? costq : nullptr, q, (const float *)ws, npx, D, dmin, dstep, st);
+}
+
 } // namespace k
 } // namespace cnncrf

@@ -47,6 +47,13 @@ void cnncrf::k::slackprop_set_costq(cnncrf_slackprop *sp, const void *costq, Una
     if (sp) sp->costq = costq, sp->q = q;
 }
 
+int cnncrf::k::slackprop_quadfit(cnncrf_slackprop *sp, float *u, float dmin, float dstep)
+{
+    if (!sp || !u) return fail(CNNCRF_EINVAL, "null argument");
+    if (!sp->ran || sp->ops.total_it <= 0) return fail(CNNCRF_ESTATE, "slackprop: get_C1 before execute");
+    return k::crf_quadfit(u, sp->cost, sp->ws.get(), (long)sp->W * sp->H, sp->D, dmin, dstep, sp->st, sp->costq, sp->q);
+}
+
 extern "C" {
 
 int cnncrf_set_conv_pairs(int enable)

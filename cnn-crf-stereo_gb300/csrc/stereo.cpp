@@ -405,9 +405,8 @@ int cnncrf_stereo_fuse_quad_fit_direct(cnncrf_stereo_t s)
     clear_error();
     if (!s) return fail(CNNCRF_EINVAL, "null stereo");
     if (!s->solver) return fail(CNNCRF_ESTATE, "fuseQuadFitDirect needs a computeSlackPropagation first");
-    float *c1 = nullptr;
-    CNNCRF_TRY(cnncrf_slackprop_get_c1(s->solver, &c1)); // solver->get_C1() (stereo/stereo.cpp:408)
-    return k::quadfit_direct(s->out.as<float>(), c1, (long)s->W * s->H, s->depth, s->dmin, s->dstep, s->st);
+    // the parabola on solver->get_C1() (stereo/stereo.cpp:408)
+    return k::slackprop_quadfit(s->solver, s->out.as<float>(), s->dmin, s->dstep);
 }
 
 int cnncrf_stereo_compute_argmax(cnncrf_stereo_t s, int lr)
