@@ -4,17 +4,20 @@
 // The reference runs every iteration as three full-image passes: a copy
 // u_ = u, ttvqf_primal_kernel (stereo/stereo.cu:701-729) and
 // thuberqf_dual_kernel (stereo/stereo.cu:773-796).  Here one launch runs K
-// iterations on a 64 x 32 pixel tile held on chip: each thread keeps four
-// pixels' u, the fit's per-pixel constants, the weights and p, q in registers, and the
-// values that neighbours read -- p.x - q.x, p.y - q.y (the primal's
-// divergence) and u_ (the dual's gradient) -- go through shared memory.  The
-// primal at (x, y) reads (x-1, y) and (x, y-1); the dual reads (x+1, y) and
-// (x, y+1), so a tile's edge corrupts one more ring of pixels per iteration:
-// the tile overlaps its neighbours by a halo of K pixels on every side and
-// writes only its interior (64 - 2K) x (32 - 2K) block.  Neighbour indices
-// are clamped to the image exactly as the reference's clamp-addressed
-// texture reads are, so tiles on the image border see the same values as the
-// unfused kernels.
+// iterations on a 64 x 32 pixel tile held on chip.  A warp has two rows, a
+// lane two columns of them: each thread keeps its 2 x 2 pixels' u, the fit's
+// per-pixel constants, the weights and p, q in registers.  The values
+// neighbours read -- p.x - q.x, p.y - q.y (the primal's divergence) and u_
+// (the dual's gradient) -- come from the thread itself, from the next lane by
+// a shuffle per row, or from the next warp through shared memory, one row of
+// each per warp.  The primal at (x, y) reads (x-1, y) and (x, y-1); the dual
+// reads (x+1, y) and (x, y+1), so a tile's edge corrupts one more ring of
+// pixels per iteration: the tile overlaps its neighbours by a halo of K pixels
+// on every side and writes only its interior (64 - 2K) x (32 - 2K) block.
+// Neighbour indices are clamped to the image exactly as the reference's
+// clamp-addressed texture reads are (EDGE tiles; the others touch no image
+// border), so tiles on the image border see the same values as the unfused
+// kernels.
 //
 // Tiles read the state (u, p, q) of the previous launch and write a second
 // copy (a workspace ping-pong), since a tile's halo belongs to other tiles.
@@ -24,6 +27,13 @@
 // per-pixel constants of the primal update are the same operations hoisted
 // out of the iteration loop, so the results equal both the CPU oracle and the
 // reference's own kernels bit for bit.  Compiled with --fmad=false.
+//
+// Bound by instruction issue: three IEEE divisions, two prox operators and
+// the clamps per pixel and iteration, on 1.7 times the interior's pixels at K
+// = 5.  Ten iterations on 4096 x 2160: 787 -> 516 us (a thread had four pixels
+// eight rows apart, every neighbour through shared memory with clamped
+// indices).  Larger tiles lose to their barriers what they save in halo: 64 x
+// 64 539 us, 64 x 48 566 us.
 #include "common.h"
 #include "kernels.h"
 
@@ -32,18 +42,20 @@ namespace k {
 
 namespace {
 
-constexpr int TX = 64, TY = 32, NT = 512, RS = NT / TX, RPT = TY / RS; // 4 rows per thread, 8 rows apart
-constexpr int KMAX = 8;                                         // iterations per launch
+constexpr int TX = 64, TY = 32, NT = 512; // a warp: 2 rows; a lane: 2 columns of them
+// Iterations per launch: a launch of K costs about 22 K (64 32) / ((64 - 2K) (32 - 2K)) + 68 us on 4096 x 2160 (the halo's
+// recomputation, the state's bytes), so 5 + 5 beat one launch of 8 or more and equal 4 + 3 + 3.
+constexpr int KMAX = 5;
 
 __device__ __forceinline__ float clampf(float v, float lo, float hi) { return fmaxf(lo, fminf(v, hi)); }
-__device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
-// prox_p with alpha = 0 (stereo/stereo.cu:752-757)
-__device__ __forceinline__ float prox_p0(float v, float beta, float sigma, float w)
+// prox_p with alpha = 0 (stereo/stereo.cu:752-757): v itself where |v| <= 0 w, else the shrunk |v| with v's sign,
+// clamped.  With beta >= 0 the first case needs no test of its own: a zero shrinks to a zero of its sign
+template <bool BETA_POS> __device__ __forceinline__ float prox_p0(float v, float beta, float sigma, float w)
 {
-    if (fabsf(v) <= __fmul_rn(w, 0.0f)) return v;
-    float m = fmaxf(0.0f, __fmaf_rn(-sigma, beta, fabsf(v)));
-    float r = __fmul_rn(m, v > 0.0f ? 1.0f : -1.0f);
+    if (!BETA_POS && fabsf(v) <= __fmul_rn(w, 0.0f)) return v;
+    const float m = fmaxf(0.0f, __fmaf_rn(-sigma, beta, fabsf(v)));
+    const float r = BETA_POS ? copysignf(m, v) : __fmul_rn(m, v > 0.0f ? 1.0f : -1.0f);
     return clampf(r, -w, w);
 }
 
@@ -60,101 +72,129 @@ struct TvArgs {
     float tau, sigma, half, C, eps;
 };
 
-__global__ void __launch_bounds__(NT, 2) k_tv_fused(const TvArgs a)
+// the K iterations of a tile whose first pixel is (ex, ey)
+template <bool EDGE, bool BETA_POS>
+__device__ __forceinline__ void tv_tile(const TvArgs &a, int ex, int ey, float2 (*sY)[TX / 2], float2 (*sU)[TX / 2])
 {
-    __shared__ float sX[TY][TX], sY[TY][TX], sU[TY][TX];
     const int W = a.W, H = a.H, K = a.K;
-    const int c = threadIdx.x & (TX - 1), r0 = threadIdx.x / TX;
-    const int ex = blockIdx.x * (TX - 2 * K) - K, ey = blockIdx.y * (TY - 2 * K) - K;
-    const int gx = ex + c;
-    const bool colin = gx >= 0 && gx < W;
-    // left / right neighbour columns: clamped to the image, then to the tile
-    // (a clamp to the tile only happens at the tile's edge, inside the halo)
-    const int cm = clampi((gx > 0 ? gx - 1 : 0) - ex, 0, TX - 1);
-    const int cp = clampi((gx + 1 < W ? gx + 1 : W - 1) - ex, 0, TX - 1);
+    const int lane = threadIdx.x & 31, wr = threadIdx.x >> 5;
+    const int gx0 = ex + 2 * lane, gy0 = ey + 2 * wr;
+    const int wm = wr > 0 ? wr - 1 : 0, wp = wr + 1 < TY / 2 ? wr + 1 : wr; // the warps above and below
 
-    // per pixel: the state (u, u_, p, q) and the primal's per-pixel constants,
-    // computed once per launch with the operations the reference applies per
-    // iteration: inner = a - b u0, den = 1 + tau b, the box u0 -+ step / 2
-    float u[RPT], ub[RPT], px[RPT], py[RPT], qx[RPT], qy[RPT];
-    float inn[RPT], den[RPT], lo[RPT], hi[RPT], wxr[RPT], wyr[RPT];
+    // per pixel (row i, column j): the state (u, u_, p, q) and the primal's per-pixel constants, computed once per
+    // launch with the operations the reference applies per iteration: inner = a - b u0, den = 1 + tau b, the box
+    // u0 -+ step / 2
+    float u[2][2], ub[2][2], px[2][2], py[2][2], qx[2][2], qy[2][2];
+    float inn[2][2], den[2][2], lo[2][2], hi[2][2], wx[2][2], wy[2][2];
 #pragma unroll
-    for (int j = 0; j < RPT; ++j) {
-        const int r = r0 + RS * j, gy = ey + r;
-        float uz = 0.0f, fa = 0.0f, fb = 0.0f;
-        u[j] = wxr[j] = wyr[j] = px[j] = py[j] = qx[j] = qy[j] = ub[j] = 0.0f;
-        if (colin && gy >= 0 && gy < H) {
-            const long i = (long)gy * W + gx;
-            u[j] = a.u_in[i];
-            uz = a.u0[i];
-            const float2 f = a.qf[i];
-            fa = f.x, fb = f.y;
-            wxr[j] = a.wx[i], wyr[j] = a.wy[i];
-            if (a.p_in) {
-                const float2 pp = a.p_in[i], qq = a.q_in[i];
-                px[j] = pp.x, py[j] = pp.y, qx[j] = qq.x, qy[j] = qq.y;
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int gx = gx0 + j, gy = gy0 + i;
+            float uz = 0.0f, fa = 0.0f, fb = 0.0f;
+            u[i][j] = wx[i][j] = wy[i][j] = px[i][j] = py[i][j] = qx[i][j] = qy[i][j] = ub[i][j] = 0.0f;
+            if (!EDGE || (gx >= 0 && gx < W && gy >= 0 && gy < H)) {
+                const long o = (long)gy * W + gx;
+                u[i][j] = a.u_in[o];
+                uz = a.u0[o];
+                const float2 f = a.qf[o];
+                fa = f.x, fb = f.y;
+                wx[i][j] = a.wx[o], wy[i][j] = a.wy[o];
+                if (a.p_in) {
+                    const float2 pp = a.p_in[o], qq = a.q_in[o];
+                    px[i][j] = pp.x, py[i][j] = pp.y, qx[i][j] = qq.x, qy[i][j] = qq.y;
+                }
             }
+            inn[i][j] = __fmaf_rn(-fb, uz, fa);
+            den[i][j] = __fmaf_rn(a.tau, fb, 1.0f);
+            lo[i][j] = __fsub_rn(uz, a.half);
+            hi[i][j] = __fadd_rn(uz, a.half);
         }
-        inn[j] = __fmaf_rn(-fb, uz, fa);
-        den[j] = __fmaf_rn(a.tau, fb, 1.0f);
-        lo[j] = __fsub_rn(uz, a.half);
-        hi[j] = __fadd_rn(uz, a.half);
-        sX[r][c] = __fsub_rn(px[j], qx[j]);
-        sY[r][c] = __fsub_rn(py[j], qy[j]);
-    }
+    const float dd = __fmaf_rn(a.sigma, a.eps, 1.0f);
+    // the row below this warp's reads its lower row's p.y - q.y
+    auto put_y = [&]() { sY[wr][lane] = make_float2(__fsub_rn(py[1][0], qy[1][0]), __fsub_rn(py[1][1], qy[1][1])); };
+    put_y();
     __syncthreads();
 
+#pragma unroll 1
     for (int it = 0; it < K; ++it) {
         // ---- primal (ttvqf_primal_kernel); u_ = u at the iteration's start
+        const float2 above = sY[wm][lane];
+        float X[2][2], Y[2][2];
 #pragma unroll
-        for (int j = 0; j < RPT; ++j) {
-            const int r = r0 + RS * j, gy = ey + r;
-            const int rm = clampi((gy > 0 ? gy - 1 : 0) - ey, 0, TY - 1);
-            const float Px = __fsub_rn(px[j], qx[j]), Py = __fsub_rn(py[j], qy[j]);
-            const float X = sX[r][cm], Y = sY[rm][c];
-            const float div = __fsub_rn(__fadd_rn(__fsub_rn(Px, X), Py), Y);
-            float un = __fmaf_rn(a.tau, div, u[j]);
-            const float num = __fmaf_rn(-a.tau, inn[j], un);
-            un = clampf(__fdiv_rn(num, den[j]), lo[j], hi[j]);
-            ub[j] = __fsub_rn(__fmul_rn(2.0f, un), u[j]);
-            u[j] = un;
-            sU[r][c] = ub[j];
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                X[i][j] = __fsub_rn(px[i][j], qx[i][j]), Y[i][j] = __fsub_rn(py[i][j], qy[i][j]);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float left = __shfl_up_sync(0xffffffffu, X[i][1], 1);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                float xl = j ? X[i][0] : left, yu = i ? Y[0][j] : (j ? above.y : above.x);
+                if (EDGE) {
+                    if (gx0 + j <= 0) xl = X[i][j];
+                    if (gy0 + i <= 0) yu = Y[i][j];
+                }
+                const float div = __fsub_rn(__fadd_rn(__fsub_rn(X[i][j], xl), Y[i][j]), yu);
+                float un = __fmaf_rn(a.tau, div, u[i][j]);
+                const float num = __fmaf_rn(-a.tau, inn[i][j], un);
+                un = clampf(__fdiv_rn(num, den[i][j]), lo[i][j], hi[i][j]);
+                ub[i][j] = __fmaf_rn(2.0f, un, -u[i][j]); // 2 un is exact
+                u[i][j] = un;
+            }
         }
+        sU[wr][lane] = make_float2(ub[0][0], ub[0][1]); // the warp above reads this warp's upper row
         __syncthreads();
         // ---- dual (thuberqf_dual_kernel), Huber parameter eps
-        const float dd = __fmaf_rn(a.sigma, a.eps, 1.0f);
+        const float2 below = sU[wp][lane];
 #pragma unroll
-        for (int j = 0; j < RPT; ++j) {
-            const int r = r0 + RS * j, gy = ey + r;
-            const int rp = clampi((gy + 1 < H ? gy + 1 : H - 1) - ey, 0, TY - 1);
-            const float uc = ub[j];
-            const float dx = __fsub_rn(sU[r][cp], uc);
-            const float dy = __fsub_rn(sU[rp][c], uc);
-            const float pnx = __fmaf_rn(a.sigma, dx, px[j]), pny = __fmaf_rn(a.sigma, dy, py[j]);
-            const float qnx = __fmaf_rn(a.sigma, dx, qx[j]), qny = __fmaf_rn(a.sigma, dy, qy[j]);
-            px[j] = clampf(__fdiv_rn(pnx, dd), -wxr[j], wxr[j]);
-            py[j] = clampf(__fdiv_rn(pny, dd), -wyr[j], wyr[j]);
-            qx[j] = prox_p0(qnx, a.C, a.sigma, wxr[j]);
-            qy[j] = prox_p0(qny, a.C, a.sigma, wyr[j]);
-            // the primals of this iteration read sX / sY before the barrier above
-            sX[r][c] = __fsub_rn(px[j], qx[j]);
-            sY[r][c] = __fsub_rn(py[j], qy[j]);
+        for (int i = 0; i < 2; ++i) {
+            const float right = __shfl_down_sync(0xffffffffu, ub[i][0], 1);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const float uc = ub[i][j];
+                float ur = j ? right : ub[i][1], ud = i ? (j ? below.y : below.x) : ub[1][j];
+                if (EDGE) {
+                    if (gx0 + j >= W - 1) ur = uc;
+                    if (gy0 + i >= H - 1) ud = uc;
+                }
+                const float dx = __fsub_rn(ur, uc), dy = __fsub_rn(ud, uc);
+                const float pnx = __fmaf_rn(a.sigma, dx, px[i][j]), pny = __fmaf_rn(a.sigma, dy, py[i][j]);
+                const float qnx = __fmaf_rn(a.sigma, dx, qx[i][j]), qny = __fmaf_rn(a.sigma, dy, qy[i][j]);
+                px[i][j] = clampf(__fdiv_rn(pnx, dd), -wx[i][j], wx[i][j]);
+                py[i][j] = clampf(__fdiv_rn(pny, dd), -wy[i][j], wy[i][j]);
+                qx[i][j] = prox_p0<BETA_POS>(qnx, a.C, a.sigma, wx[i][j]);
+                qy[i][j] = prox_p0<BETA_POS>(qny, a.C, a.sigma, wy[i][j]);
+            }
         }
+        put_y();         // this iteration's primals read sY before the barrier above
         __syncthreads(); // every dual has read sU before the next primal rewrites it
     }
 
     // ---- the interior block, inside the image
-    if (!colin || c < K || c >= TX - K) return;
 #pragma unroll
-    for (int j = 0; j < RPT; ++j) {
-        const int r = r0 + RS * j, gy = ey + r;
-        if (r < K || r >= TY - K || gy < 0 || gy >= H) continue;
-        const long i = (long)gy * W + gx;
-        a.u_out[i] = u[j];
-        a.p_out[i] = make_float2(px[j], py[j]);
-        a.q_out[i] = make_float2(qx[j], qy[j]);
-        if (a.ubar_out) a.ubar_out[i] = ub[j];
-    }
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int c = 2 * lane + j, r = 2 * wr + i, gx = gx0 + j, gy = gy0 + i;
+            if (c < K || c >= TX - K || r < K || r >= TY - K) continue;
+            if (EDGE && (gx < 0 || gx >= W || gy < 0 || gy >= H)) continue;
+            const long o = (long)gy * W + gx;
+            a.u_out[o] = u[i][j];
+            a.p_out[o] = make_float2(px[i][j], py[i][j]);
+            a.q_out[o] = make_float2(qx[i][j], qy[i][j]);
+            if (a.ubar_out) a.ubar_out[o] = ub[i][j];
+        }
+}
+
+template <bool BETA_POS> __global__ void __launch_bounds__(NT, 2) k_tv_fused(const TvArgs a)
+{
+    __shared__ float2 sY[TY / 2][TX / 2], sU[TY / 2][TX / 2];
+    const int ex = blockIdx.x * (TX - 2 * a.K) - a.K, ey = blockIdx.y * (TY - 2 * a.K) - a.K;
+    // pixels 0 and W - 1 (H - 1) are the only ones whose neighbours are clamped
+    if (ex > 0 && ey > 0 && ex + TX < a.W && ey + TY < a.H) tv_tile<false, BETA_POS>(a, ex, ey, sY, sU);
+    else tv_tile<true, BETA_POS>(a, ex, ey, sY, sU);
 }
 
 struct TvWs {
@@ -233,7 +273,8 @@ int tv_iterate(float *u, float *u_, const float *u0, const float *qf, float *p, 
         const dim3 grid(ceil_div(W, TX - 2 * K), ceil_div(H, TY - 2 * K));
         {
             CNNCRF_PROF("tv", st);
-            k_tv_fused<<<grid, NT, 0, st>>>(a);
+            if (C >= 0.0f) k_tv_fused<true><<<grid, NT, 0, st>>>(a);
+            else k_tv_fused<false><<<grid, NT, 0, st>>>(a);
         }
         CNNCRF_CHECK_LAUNCH();
         in_set = out_set;
