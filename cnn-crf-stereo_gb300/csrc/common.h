@@ -99,6 +99,7 @@ class Prof {
     cudaStream_t st_;
     cudaEvent_t a_ = nullptr;
 };
+bool profiling(); // launches are being timed
 #define CNNCRF_PROF(name, st) ::cnncrf::Prof prof__(name, st)
 
 // An NVTX range around a whole stage of an API call (the volume, the CRF,

@@ -1,6 +1,8 @@
 // k_front.cu -- mirror padding and RGB normalisation (the front end of
 // ColorStereoNet::predict).  Compiled with --fmad=false: results must match
 // the CPU oracle bit for bit.
+#include <algorithm>
+
 #include "common.h"
 #include "kernels.h"
 
@@ -29,14 +31,26 @@ __global__ void k_pad(const float4 *__restrict__ in, int W, int H, int p, float4
     out[i] = in[(long)mirror_idx(y - p, H) * W + mirror_idx(x - p, W)];
 }
 
-// value of plane c at pixel i: RGB channel, or rgb_to_gray_kernel's weights
+// plane c of a pixel: RGB channel, or rgb_to_gray_kernel's weights
 // (stereo/stereo.cu:853-863) evaluated in double and rounded once.
-__device__ __forceinline__ float plane_val(const float *rgba, long i, int c, int gray)
+template <bool GRAY> __device__ __forceinline__ float plane_val(const float4 &px, int c)
 {
-    const float *px = rgba + 4 * i;
-    if (gray)
-        return (float)(0.2989 * (double)px[0] + 0.5870 * (double)px[1] + 0.1140 * (double)px[2]);
-    return px[c];
+    if (GRAY) return (float)(0.2989 * (double)px.x + 0.5870 * (double)px.y + 0.1140 * (double)px.z);
+    return c == 0 ? px.x : (c == 1 ? px.y : px.z);
+}
+
+// a caller's image may start on any float
+template <bool AL> __device__ __forceinline__ float4 load_px(const float4 *p)
+{
+    if (AL) return __ldg(p);
+    const float *f = (const float *)p;
+    return make_float4(__ldg(f), __ldg(f + 1), __ldg(f + 2), 0.0f);
+}
+
+// image i of the batch: the first n from a, the others from b
+__device__ __forceinline__ const float4 *image(const float4 *a, const float4 *b, int n, int i, long npx)
+{
+    return i < n ? a + i * npx : b + (i - n) * npx;
 }
 
 // FP64 sums in a fixed order shared with the CPU oracle: lane j of a warp sums
@@ -49,69 +63,108 @@ __device__ __forceinline__ double warp_tree_sum(double s)
     return s;
 }
 
-// One warp per (plane, row).  pass 0 sums the values, pass 1 the squares of
-// (v - mean_c) rounded to float.
-__global__ void k_rowsums(const float *__restrict__ rgba, int Wp, int Hp, int planes, int gray,
-                          int pass, const float *__restrict__ stats, double *__restrict__ rows)
+// The statistic of one plane from its row sums, added by one warp in the same
+// lane / butterfly order; every lane has it.  Each consumer's CTAs take it
+// from the row sums themselves: a launch between them cost 8 us
+__device__ __forceinline__ double plane_sum(const double *rows, int Hp, int lane)
 {
-    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (w >= planes * Hp) return;
-    rgba += (long)blockIdx.y * Wp * Hp * 4; // image of the batch
-    rows += (long)blockIdx.y * 3 * Hp;
-    stats += blockIdx.y * 8;
-    const int c = w / Hp, y = w - c * Hp;
-    const long base = (long)y * Wp;
     double s = 0.0;
-    if (pass == 0) {
-        for (int x = lane; x < Wp; x += 32) s += (double)plane_val(rgba, base + x, c, gray);
-    } else {
-        const float mean = stats[c];
-        for (int x = lane; x < Wp; x += 32) {
-            const float v = __fsub_rn(plane_val(rgba, base + x, c, gray), mean);
-            s += (double)__fmul_rn(v, v);
+#pragma unroll 8
+    for (int y = lane; y < Hp; y += 32) s += rows[y];
+    return warp_tree_sum(s);
+}
+
+// One warp per (row, plane), a few rows per CTA.  pass 0 sums the values,
+// pass 1 the squares of (v - mean_c) rounded to float.  rows: [image][pass][3]
+// [Hp].  Bound by the FP64 additions (conversions by integer operations took the
+// same time); the warps are small and many, their loads eight pixels ahead.
+// Both sides of a KITTI pair in three launches take 72 us, in the ten launches
+// of one side at a time with the statistics in launches of their own 107 us.
+template <bool GRAY> __host__ __device__ constexpr int row_cta() { return GRAY ? 4 : 2; }
+template <bool GRAY, bool AL>
+__global__ void __launch_bounds__(32 * row_cta<GRAY>() * (GRAY ? 1 : 3))
+    k_rowsums(const float4 *__restrict__ ia, const float4 *__restrict__ ib, int n, int Wp, int Hp, int pass,
+              double *__restrict__ rowsum)
+{
+    constexpr int NP = GRAY ? 1 : 3;
+    __shared__ float smean[NP];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int r = warp / NP, c = warp - r * NP, y = blockIdx.x * row_cta<GRAY>() + r;
+    double *rows = rowsum + (long)blockIdx.y * 6 * Hp;
+    float mean = 0.0f;
+    if (pass) {
+        if (warp < NP) {
+            const double s = plane_sum(rows + warp * Hp, Hp, lane);
+            if (lane == 0) smean[warp] = (float)(s / (double)((long)Wp * Hp));
+        }
+        __syncthreads();
+        mean = smean[c];
+        rows += 3 * Hp;
+    }
+    if (y >= Hp) return;
+    const float4 *px = image(ia, ib, n, blockIdx.y, (long)Wp * Hp) + (long)y * Wp;
+    double s = 0.0;
+#pragma unroll 8
+    for (int x = lane; x < Wp; x += 32) {
+        float v = plane_val<GRAY>(load_px<AL>(px + x), c);
+        if (pass) v = __fsub_rn(v, mean), v = __fmul_rn(v, v);
+        s += (double)v;
+    }
+    s = warp_tree_sum(s);
+    if (lane == 0) rows[c * Hp + y] = s;
+}
+
+// (v - mean) / population std, and the coordinate planes.  A CTA takes the
+// statistics once, so the grid is a few CTAs per SM however large the images.
+template <bool GRAY, bool AL>
+__global__ void __launch_bounds__(256)
+    k_norm_write(const float4 *__restrict__ ia, const float4 *__restrict__ ib, int n, int Wp, int Hp, int ic,
+                 const double *__restrict__ rowsum, float *__restrict__ out)
+{
+    constexpr int NP = GRAY ? 1 : 3;
+    __shared__ float stats[2][3];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long npx = (long)Wp * Hp;
+    const double *rows = rowsum + (long)blockIdx.y * 6 * Hp;
+    if (warp < 2 * NP) {
+        const int k = warp / NP, c = warp - k * NP;
+        const double s = plane_sum(rows + (3 * k + c) * Hp, Hp, lane) / (double)npx;
+        if (lane == 0) stats[k][c] = (float)(k ? sqrt(s) : s);
+    }
+    __syncthreads();
+    const float4 *px = image(ia, ib, n, blockIdx.y, npx);
+    out += (long)blockIdx.y * npx * ic;
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < npx; i += (long)gridDim.x * blockDim.x) {
+        const float4 p = load_px<AL>(px + i);
+#pragma unroll
+        for (int c = 0; c < NP; ++c) {
+            const float v = __fsub_rn(plane_val<GRAY>(p, c), stats[0][c]), sd = stats[1][c];
+            out[i * ic + c] = sd > 0.0f ? __fdiv_rn(v, sd) : 0.0f;
+        }
+        if (ic == 5) { // stereo/colorstereonet.cpp:102-121
+            const int y = (int)(i / Wp), x = (int)(i - (long)y * Wp);
+            out[i * ic + 3] = (float)(((double)x - (double)Wp / 2.0) / (double)Wp);
+            out[i * ic + 4] = (float)(((double)y - (double)Hp / 2.0) / (double)Hp);
         }
     }
-    s = warp_tree_sum(s);
-    if (lane == 0) rows[w] = s;
 }
 
-// One warp per plane: the row sums in the same lane / butterfly order -> mean
-// (pass 0) or population std (pass 1).
-__global__ void k_finalize(const double *__restrict__ rows, int Hp, int planes, long N, int pass,
-                           float *__restrict__ stats)
+template <bool GRAY, bool AL>
+int launch_normalize(const float4 *a, const float4 *b, int n, int nimg, int Wp, int Hp, int ic, float *out, double *rows,
+                     cudaStream_t st)
 {
-    const int c = blockIdx.x, lane = threadIdx.x;
-    rows += (long)blockIdx.y * 3 * Hp;
-    stats += blockIdx.y * 8;
-    double s = 0.0;
-    for (int y = lane; y < Hp; y += 32) s += rows[c * Hp + y];
-    s = warp_tree_sum(s);
-    if (lane == 0) {
-        if (pass == 0) stats[c] = (float)(s / (double)N);
-        else stats[4 + c] = (float)sqrt(s / (double)N);
+    const long npx = (long)Wp * Hp;
+    for (int pass = 0; pass < 2; ++pass) {
+        CNNCRF_PROF("rowsums", st);
+        k_rowsums<GRAY, AL><<<dim3(ceil_div(Hp, row_cta<GRAY>()), nimg), 32 * row_cta<GRAY>() * (GRAY ? 1 : 3), 0, st>>>(a, b, n, Wp, Hp, pass, rows);
     }
-}
-
-__global__ void k_norm_write(const float *__restrict__ rgba, int Wp, int Hp, int ic,
-                             const float *__restrict__ stats, float *__restrict__ out)
-{
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long)Wp * Hp) return;
-    rgba += (long)blockIdx.y * Wp * Hp * 4;
-    stats += blockIdx.y * 8;
-    out += (long)blockIdx.y * Wp * Hp * ic;
-    int gray = ic == 1;
-    int planes = gray ? 1 : 3;
-    for (int c = 0; c < planes; ++c) {
-        float v = __fsub_rn(plane_val(rgba, i, c, gray), stats[c]);
-        float sd = stats[4 + c];
-        out[i * ic + c] = sd > 0.0f ? __fdiv_rn(v, sd) : 0.0f;
+    {
+        CNNCRF_PROF("norm_write", st);
+        const long ctas = std::min<long>(ceil_div(npx, 256), std::max(8, ceil_div(608, nimg))); // 4 per SM
+        k_norm_write<GRAY, AL><<<dim3((unsigned)ctas, nimg), 256, 0, st>>>(a, b, n, Wp, Hp, ic, rows, out);
     }
-    if (ic == 5) { // stereo/colorstereonet.cpp:102-121
-        int y = (int)(i / Wp), x = (int)(i - (long)y * Wp);
-        out[i * ic + 3] = (float)(((double)x - (double)Wp / 2.0) / (double)Wp);
-        out[i * ic + 4] = (float)(((double)y - (double)Hp / 2.0) / (double)Hp);
-    }
+    CNNCRF_CHECK_LAUNCH();
+    return CNNCRF_OK;
 }
 
 } // namespace
@@ -127,37 +180,17 @@ int pad_rgba(const float *in, int W, int H, int p, float *out, cudaStream_t st, 
     return CNNCRF_OK;
 }
 
-size_t normalize_scratch_bytes(int Hp, int nimg) { return (sizeof(double) * 3 * (size_t)Hp + 32) * nimg + 64; }
+size_t normalize_scratch_bytes(int Hp, int nimg) { return sizeof(double) * 6 * (size_t)Hp * nimg; }
 
-int normalize(const float *rgba, int Wp, int Hp, int ic, float *out, void *scratch, cudaStream_t st, int nimg)
+int normalize(const float *rgba, const float *rgba2, int Wp, int Hp, int ic, float *out, void *scratch, cudaStream_t st,
+              int nimg)
 {
-    int gray = ic == 1, planes = gray ? 1 : 3;
-    double *rows = (double *)scratch;
-    float *stats = (float *)((char *)scratch + sizeof(double) * 3 * (size_t)Hp * nimg);
-    long N = (long)Wp * Hp;
-    const long nthreads = 32L * planes * Hp;
-    {
-        CNNCRF_PROF("rowsums", st);
-        k_rowsums<<<dim3(ceil_div(nthreads, 256), nimg), 256, 0, st>>>(rgba, Wp, Hp, planes, gray, 0, stats, rows);
-    }
-    {
-        CNNCRF_PROF("finalize", st);
-        k_finalize<<<dim3(planes, nimg), 32, 0, st>>>(rows, Hp, planes, N, 0, stats);
-    }
-    {
-        CNNCRF_PROF("rowsums", st);
-        k_rowsums<<<dim3(ceil_div(nthreads, 256), nimg), 256, 0, st>>>(rgba, Wp, Hp, planes, gray, 1, stats, rows);
-    }
-    {
-        CNNCRF_PROF("finalize", st);
-        k_finalize<<<dim3(planes, nimg), 32, 0, st>>>(rows, Hp, planes, N, 1, stats);
-    }
-    {
-        CNNCRF_PROF("norm_write", st);
-        k_norm_write<<<dim3(ceil_div(N, 256), nimg), 256, 0, st>>>(rgba, Wp, Hp, ic, stats, out);
-    }
-    CNNCRF_CHECK_LAUNCH();
-    return CNNCRF_OK;
+    const float4 *a = (const float4 *)rgba, *b = (const float4 *)rgba2;
+    const int total = rgba2 ? 2 * nimg : nimg;
+    const bool al = (((uintptr_t)rgba | (uintptr_t)rgba2) & 15) == 0;
+    auto *launch = ic == 1 ? (al ? launch_normalize<true, true> : launch_normalize<true, false>)
+                           : (al ? launch_normalize<false, true> : launch_normalize<false, false>);
+    return launch(a, b, nimg, total, Wp, Hp, ic, out, (double *)scratch, st);
 }
 
 } // namespace k

@@ -16,10 +16,10 @@ namespace k {
 int pad_rgba(const float *in, int W, int H, int p, float *out, cudaStream_t st, int nimg = 1);
 // zero-mean / unit-std planes of a padded RGBA image -> NHWC [Hp][Wp][ic]
 // (stereo/colorstereonet.cpp:53-64,102-121; stereo/utils.cu:169-237).
-// scratch: >= 6*Hp doubles + 8 floats.
-// images of a batch are contiguous ([nimg][Hp][Wp][4] in, [nimg][Hp][Wp][ic] out)
-int normalize(const float *rgba, int Wp, int Hp, int ic, float *out, void *scratch,
-              cudaStream_t st, int nimg = 1);
+// images of a batch are contiguous ([nimg][Hp][Wp][4] in, [nimg][Hp][Wp][ic] out); with rgba2 as well, its nimg images
+// follow those of rgba in out.  scratch: normalize_scratch_bytes of all images
+int normalize(const float *rgba, const float *rgba2, int Wp, int Hp, int ic, float *out, void *scratch, cudaStream_t st,
+              int nimg = 1);
 size_t normalize_scratch_bytes(int Hp, int nimg = 1);
 
 // ------------------------------------------------------------ FP32 conv

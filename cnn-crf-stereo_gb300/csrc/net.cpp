@@ -201,51 +201,82 @@ int cnncrf_net::set_disparities(float mn, float mx, float step, float *d_out)
     return CNNCRF_OK;
 }
 
-int cnncrf_net::pairwise_fp32()
+int cnncrf_net::pairwise_fp32(cudaStream_t q)
 {
     // crop by pad-2 of the normalised left image (stereo/colorstereonet.cpp:69-73)
     int cr = pad - 2, ic = d.in_channels, P = d.pw_channels;
-    const float *in = norm[0].as<float>() + ((size_t)cr * w + cr) * ic;
+    const float *in = norm_side(0) + ((size_t)cr * w + cr) * ic;
     k::ConvArgs a1{in, H + 4, W + 4, pw[0].cin, (long)ic, (long)w * ic, pw[0].wt.as<float>(),
                    pw[0].bias.as<float>(), pw[0].cout, 3, 3, 1, pwa.as<float>()};
     a1.n_img = n, a1.in_img = (long)h * w * ic, a1.out_img = (long)(H + 2) * (W + 2) * P;
-    CNNCRF_TRY(k::conv_simt(a1, st));
+    CNNCRF_TRY(k::conv_simt(a1, q));
     k::ConvArgs a2{pwa.as<float>(), H + 2, W + 2, pw[1].cin, (long)pw[1].cin, (long)(W + 2) * pw[1].cin,
                    pw[1].wt.as<float>(), pw[1].bias.as<float>(), pw[1].cout, 3, 3, 1, pwb.as<float>()};
     a2.n_img = n, a2.in_img = (long)(H + 2) * (W + 2) * P, a2.out_img = (long)H * W * P;
-    CNNCRF_TRY(k::conv_simt(a2, st));
-    return k::conv_head2(pwb.as<float>(), H * W, pw[2].cin, pw[2].wt.as<float>(), pwout, st, n);
+    CNNCRF_TRY(k::conv_simt(a2, q));
+    return k::conv_head2(pwb.as<float>(), H * W, pw[2].cin, pw[2].wt.as<float>(), pwout, q, n);
+}
+
+// the feature layers of one side, from its half of norm
+int cnncrf_net::features_fp32(int s, cudaStream_t q)
+{
+    const float *cur = norm_side(s);
+    int ch = h, cw = w, cc = d.in_channels;
+    for (size_t l = 0; l < feat.size(); ++l) {
+        Layer &L = feat[l];
+        float *out = act[s][l & 1].as<float>();
+        k::ConvArgs a{cur, ch, cw, cc, (long)cc, (long)cw * cc, L.wt.as<float>(), L.bias.as<float>(),
+                      L.cout, L.kh, L.kw, L.act, out};
+        int oh = ch - (L.kh - 1), ow = cw - (L.kw - 1);
+        a.n_img = n, a.in_img = (long)ch * cw * cc, a.out_img = (long)oh * ow * L.cout;
+        CNNCRF_TRY(k::conv_simt(a, q));
+        ch = oh, cw = ow, cc = L.cout;
+        cur = out;
+    }
+    feats[s] = const_cast<float *>(cur);
+    if (d.unary == CNNCRF_UNARY_ONE_MINUS_DOT) return k::l2norm(feats[s], (long)H * W * n, d.feat_channels, q);
+    return CNNCRF_OK;
+}
+
+int cnncrf_net::make_side_stream()
+{
+    int prio = 0;
+    CNNCRF_CUDA(cudaStreamGetPriority(st, &prio));
+    if (!side_st) CNNCRF_CUDA(cudaStreamCreateWithPriority(&side_st, cudaStreamNonBlocking, prio));
+    if (!fork_ev) CNNCRF_CUDA(cudaEventCreateWithFlags(&fork_ev, cudaEventDisableTiming));
+    if (!join_ev) CNNCRF_CUDA(cudaEventCreateWithFlags(&join_ev, cudaEventDisableTiming));
+    return CNNCRF_OK;
 }
 
 int cnncrf_net::predict_fp32(const float *left, const float *right, bool reuse_left_features)
 {
-    const float *img[2] = {left, right};
-    int ic = d.in_channels;
-    const bool reuse = reuse_left_features && left_ok;
+    const int ic = d.in_channels;
+    const bool reuse = reuse_left_features && left_ok; // feats[0] and the left half of norm still hold this input's
     left_ok = false;
-    for (int s = 0; s < 2; ++s) {
-        if (s == 0 && reuse) continue; // feats[0] and norm[0] still hold this input's features
-        CNNCRF_TRY(k::normalize(img[s], w, h, ic, norm[s].as<float>(), scratch.get(), st, n));
-        const float *cur = norm[s].as<float>();
-        int ch = h, cw = w, cc = ic;
-        for (size_t l = 0; l < feat.size(); ++l) {
-            Layer &L = feat[l];
-            float *out = act[s][l & 1].as<float>();
-            k::ConvArgs a{cur, ch, cw, cc, (long)cc, (long)cw * cc, L.wt.as<float>(), L.bias.as<float>(),
-                          L.cout, L.kh, L.kw, L.act, out};
-            int oh = ch - (L.kh - 1), ow = cw - (L.kw - 1);
-            a.n_img = n, a.in_img = (long)ch * cw * cc, a.out_img = (long)oh * ow * L.cout;
-            CNNCRF_TRY(k::conv_simt(a, st));
-            ch = oh, cw = ow, cc = L.cout;
-            cur = out;
-        }
-        feats[s] = const_cast<float *>(cur);
-        if (d.unary == CNNCRF_UNARY_ONE_MINUS_DOT)
-            CNNCRF_TRY(k::l2norm(feats[s], (long)H * W * n, d.feat_channels, st));
+    if (reuse) CNNCRF_TRY(k::normalize(right, nullptr, w, h, ic, norm_side(1), scratch.get(), st, n));
+    else CNNCRF_TRY(k::normalize(left, right, w, h, ic, norm_side(0), scratch.get(), st, n));
+    // Two independent chains of layers, side by side: the right image's, and the left one's and the pairwise net's.  One
+    // layer of one image is a few waves of CTAs with the last of them partly empty (256 x 192: 1.4 waves); the other
+    // chain's next layer fills it.  While launches are timed they run one after the other, so that a kernel's time is
+    // its own.
+    auto left_chain = [&](cudaStream_t q) -> int {
+        if (!reuse) CNNCRF_TRY(features_fp32(0, q));
+        return d.with_pairwise ? pairwise_fp32(q) : CNNCRF_OK;
+    };
+    if (profiling() || (reuse && !d.with_pairwise)) {
+        CNNCRF_TRY(features_fp32(1, st));
+        CNNCRF_TRY(left_chain(st));
+    } else {
+        CNNCRF_CUDA(cudaEventRecord(fork_ev, st));
+        CNNCRF_CUDA(cudaStreamWaitEvent(side_st, fork_ev, 0));
+        const int rc1 = features_fp32(1, side_st);
+        const int rc0 = rc1 == CNNCRF_OK ? left_chain(st) : rc1;
+        CNNCRF_CUDA(cudaEventRecord(join_ev, side_st)); // joined after an error too
+        CNNCRF_CUDA(cudaStreamWaitEvent(st, join_ev, 0));
+        CNNCRF_TRY(rc0);
     }
     CNNCRF_TRY(k::correlation(feats[0], feats[1], H, W, d.feat_channels, d_list.as<float>(), D, omin, omax,
                               interp || force_interp, d.unary, vol, st, n, (long)H * W * d.feat_channels));
-    if (d.with_pairwise) CNNCRF_TRY(pairwise_fp32());
     left_ok = true;
     return CNNCRF_OK;
 }
@@ -263,11 +294,11 @@ int cnncrf_net::predict_concat(const float *left, const float *right)
     const long bw = w + 2, bh = h + 2;
     const long x_img = bh * bw * ic, z_img = bh * bw * C;
     for (int s = 0; s < 2; ++s) {
-        CNNCRF_TRY(k::normalize(img[s], w, h, ic, norm[s].as<float>(), scratch.get(), st, n));
+        CNNCRF_TRY(k::normalize(img[s], nullptr, w, h, ic, norm_side(s), scratch.get(), st, n));
         float *x = cx[s].as<float>(), *z = cz[s].as<float>();
         for (int i = 0; i < n; ++i)
             CNNCRF_CUDA(cudaMemcpy2DAsync(x + i * x_img + (bw + 1) * ic, sizeof(float) * bw * ic,
-                                          norm[s].as<float>() + (long)i * h * w * ic, sizeof(float) * w * ic,
+                                          norm_side(s) + (long)i * h * w * ic, sizeof(float) * w * ic,
                                           sizeof(float) * w * ic, h, cudaMemcpyDeviceToDevice, st));
         for (size_t l = 0; l < feat.size(); ++l) {
             Layer &L = feat[l];
@@ -432,7 +463,7 @@ int cnncrf_net_init(cnncrf_net_t net, float min_disp, float max_disp, float step
     if (rect_corr != 0) return fail(CNNCRF_EUNSUPPORTED, "rect_corr != 0 is not built");
     int ic = net->d.in_channels, h = net->h, w = net->w, H = net->H, W = net->W, nb = net->n;
     size_t np = (size_t)h * w * nb;
-    for (int s = 0; s < 2; ++s) CNNCRF_TRY(net->norm[s].reserve(np * ic * sizeof(float)));
+    CNNCRF_TRY(net->norm.reserve(2 * np * ic * sizeof(float)));
     size_t amax = 0;
     if (net->d.topology != CNNCRF_TOPO_CONCAT) { // valid convs: each layer shrinks the maps
         int ch = h, cw = w;
@@ -446,6 +477,7 @@ int cnncrf_net_init(cnncrf_net_t net, float min_disp, float max_disp, float step
     for (int s = 0; s < 2; ++s)
         for (int b = 0; b < 2; ++b)
             if (fp32 && !concat) CNNCRF_TRY(net->act[s][b].reserve(amax * nb * sizeof(float)));
+    if (fp32 && !concat) CNNCRF_TRY(net->make_side_stream());
     if (concat) { // the borders stay zero: predict writes only the interiors
         const size_t bpx = (size_t)(h + 2) * (w + 2) * nb, C = net->d.feat_channels;
         for (int s = 0; s < 2; ++s) {
@@ -456,7 +488,7 @@ int cnncrf_net_init(cnncrf_net_t net, float min_disp, float max_disp, float step
             CNNCRF_CUDA(cudaMemsetAsync(net->cz[s].get(), 0, bpx * C * sizeof(float), net->st));
         }
     }
-    CNNCRF_TRY(net->scratch.reserve(k::normalize_scratch_bytes(h, nb)));
+    CNNCRF_TRY(net->scratch.reserve(k::normalize_scratch_bytes(h, 2 * nb)));
     if (net->d.with_pairwise) {
         int P = net->d.pw_channels;
         if (fp32 && !concat) {

@@ -41,7 +41,9 @@ struct cnncrf_net {
     bool vol_fp32 = true;
 
     // activations
-    cnncrf::DevBuf norm[2], act[2][2], pwa, pwb, scratch;
+    cnncrf::DevBuf norm; // both sides in one buffer, left images first
+    cnncrf::DevBuf act[2][2], pwa, pwb, scratch;
+    float *norm_side(int s) const { return norm.as<float>() + (size_t)s * n * h * w * d.in_channels; }
     float *feats[2] = {nullptr, nullptr};
     bool inited = false;
     // the concatenating topology: growth rate g, the zero-bordered input
@@ -69,13 +71,27 @@ struct cnncrf_net {
     int upload(int slot);
     int predict(const float *left, const float *right);
     int predict_fp32(const float *left, const float *right, bool reuse_left);
+    int features_fp32(int side, cudaStream_t q);
+    // FP32 path: the stream of the second chain of layers that predict runs beside its own (made by init)
+    cudaStream_t side_st = nullptr;
+    cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
+    int make_side_stream();
+    cnncrf_net() = default;
+    cnncrf_net(const cnncrf_net &) = delete;
+    cnncrf_net &operator=(const cnncrf_net &) = delete;
+    ~cnncrf_net()
+    {
+        if (side_st) cudaStreamDestroy(side_st);
+        if (fork_ev) cudaEventDestroy(fork_ev);
+        if (join_ev) cudaEventDestroy(join_ev);
+    }
     // FP32 path: the next predict's left input is the last predict's (same
     // padded image): keep its left features (and normalised image) instead of
     // recomputing them.  One-shot; honoured only while left_ok.
     bool reuse_left = false;
-    bool left_ok = false; // feats[0] / norm[0] are those of the last completed FP32 predict
+    bool left_ok = false; // feats[0] / the left half of norm are those of the last completed FP32 predict
     int predict_bf16(const float *left, const float *right);
-    int pairwise_fp32();
+    int pairwise_fp32(cudaStream_t q);
     int set_disparities(float mn, float mx, float step, float *d_out);
 };
 

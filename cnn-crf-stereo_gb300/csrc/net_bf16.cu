@@ -62,17 +62,16 @@ int cnncrf_net::predict_bf16(const float *left, const float *right)
 {
     tc_calls.clear();
     if (d.num_layers < 2) return fail(CNNCRF_EUNSUPPORTED, "BF16 path needs >= 2 feature layers");
-    const float *img[2] = {left, right};
     const int ic = d.in_channels, F = d.feat_channels, cp = cp_feat;
     const size_t h1 = h - 2, w1 = w - 2;
-    for (int s = 0; s < 2; ++s) {
-        CNNCRF_TRY(k::normalize(img[s], w, h, ic, norm[s].as<float>(), scratch.get(), st, n));
+    CNNCRF_TRY(k::normalize(left, right, w, h, ic, norm_side(0), scratch.get(), st, n));
+    {
         Layer &L0 = feat[0];
-        k::ConvArgs a{norm[s].as<float>(), h, w, ic, (long)ic, (long)w * ic, L0.wt.as<float>(), L0.bias.as<float>(),
+        k::ConvArgs a{norm_side(0), h, w, ic, (long)ic, (long)w * ic, L0.wt.as<float>(), L0.bias.as<float>(),
                       F, 3, 3, 1, nullptr};
-        a.out16 = (uint16_t *)a16[0].get() + (size_t)s * n * h1 * w1 * cp;
+        a.out16 = a16[0].get();
         a.out_cs = cp;
-        a.n_img = n, a.in_img = (long)h * w * ic, a.out_img = (long)(h1 * w1 * cp);
+        a.n_img = 2 * n, a.in_img = (long)h * w * ic, a.out_img = (long)(h1 * w1 * cp); // left images, then right images
         if (k::conv_first_tc_supported(a)) CNNCRF_TRY(k::conv_first_tc(a, err.as<int>(), st));
         else CNNCRF_TRY(k::conv_simt(a, st));
     }
@@ -114,7 +113,7 @@ int cnncrf_net::predict_bf16(const float *left, const float *right)
     }
     if (d.with_pairwise) {
         int cr = pad - 2;
-        const float *in = norm[0].as<float>() + ((size_t)cr * w + cr) * ic;
+        const float *in = norm_side(0) + ((size_t)cr * w + cr) * ic;
         k::ConvArgs a1{in, H + 4, W + 4, pw[0].cin, (long)ic, (long)w * ic, pw[0].wt.as<float>(), pw[0].bias.as<float>(),
                        pw[0].cout, 3, 3, 1, nullptr};
         a1.out16 = pw16.get();

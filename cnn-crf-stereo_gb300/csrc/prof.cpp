@@ -55,6 +55,8 @@ cudaEvent_t get_event()
 }
 } // namespace
 
+bool profiling() { return g_enabled.load(std::memory_order_relaxed); }
+
 Range::Range(const char *name) { range_push(name); }
 Range::~Range() { nvtxDomainRangePop(domain()); }
 

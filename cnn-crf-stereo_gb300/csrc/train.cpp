@@ -223,7 +223,7 @@ int cnncrf_train::build()
     pool.resize(poolsz);
     for (auto &b : pool) CNNCRF_TRY(zalloc(b, lmax));
     CNNCRF_TRY(zalloc(fbuf, 2 * N * fstride() * es()));
-    CNNCRF_TRY(scratch.reserve(k::normalize_scratch_bytes(h, n)));
+    CNNCRF_TRY(scratch.reserve(k::normalize_scratch_bytes(h, 2 * n)));
     CNNCRF_TRY(vol.reserve(sizeof(float) * N * D));
     CNNCRF_TRY(zalloc(y1, (size_t)n * (H + 2) * (W + 2) * pstride() * es()));
     CNNCRF_TRY(zalloc(y2, N * pstride() * es()));
@@ -344,10 +344,8 @@ int cnncrf_train::forward(const float *l, const float *r)
 {
     const float *img[2] = {l, r};
     const int F = d.feat_channels, L = (int)feat.size();
-    for (int s = 0; s < 2; ++s) {
-        CNNCRF_TRY(k::pad_rgba(img[s], W, H, p, padded_s(s), st, n));
-        CNNCRF_TRY(k::normalize(padded_s(s), w, h, ic, norm_s(s), scratch.get(), st, n));
-    }
+    for (int s = 0; s < 2; ++s) CNNCRF_TRY(k::pad_rgba(img[s], W, H, p, padded_s(s), st, n));
+    CNNCRF_TRY(k::normalize(padded_s(0), padded_s(1), w, h, ic, norm_s(0), scratch.get(), st, n));
     if (norm16.get()) CNNCRF_TRY(k::train_to_bf16_c64(norm.as<float>(), (long)nf() * h * w, ic, norm16.get(), st));
     for (int li = 0; li < L; ++li) CNNCRF_TRY(run_layer(li)); // both sides at once
     if (!bf16) { // (the BF16 last layer's epilogue wrote the normalised features)
