@@ -301,7 +301,7 @@ __global__ void __launch_bounds__(2 * TN, 2) k_conv_nt(ConvArgs a, int Ho, int W
 // The wide layers (Cin a multiple of 16 or 20, 16-byte aligned pixels): a CTA
 // of four warps computes 128 output pixels, taken in row order across row
 // ends so that narrow images leave no part of a tile idle; lane l has pixels
-// l, l + 32, l + 64, l + 96 of it, warp w channels CPW w .. CPW w + CPW - 1.
+// l, l + 32, l + 64, l + 96 of it, warp w CPW channels (w_pitch).
 // Four k steps of a warp are four 16-byte loads of its pixels' inputs
 // (conflict-free at a pitch of 20 floats), broadcast loads of its weights and
 // 8 CPW packed fmas; every scheduler carries the same two warps.  k-slices of
@@ -310,30 +310,43 @@ __global__ void __launch_bounds__(2 * TN, 2) k_conv_nt(ConvArgs a, int Ho, int W
 // deep.  Per output the terms in ascending k, one fmaf each: the same bits as
 // k_conv_nt.
 //
-// Bound by the FMA pipe: fma.rn.f32x2 issues every 2.5 cycles (measured alone
-// 2.48 to 2.7), 130 cycles per warp and k step at CPW = 26; the 3x3 layers of
-// a 720 x 480 pair take about 155 with the epilogue.  All FP32 convolutions of
-// that pair with its re-match: 33.4 -> 24.9 ms; of a KITTI pair in 2x2 layers
-// 14.5 -> 11.5 ms; of a 256 x 192 grey pair 4.58 -> 2.93 ms (k_conv_nt: 14
-// warps per SM on four schedulers, 8 pack moves per 32 fmas, a row's last
-// tile).  Measured and left out: three CTAs at 168 registers (spills, 26.0
-// ms), scalar fmas (33.3 ms), exactly 25 channels per warp with one unpaired
-// (25.3 ms).
+// Bound by the FMA pipe: fma.rn.f32x2 issues every 2.2 cycles where it shares
+// an operand register with the one before it (else 2.5 to 3), 114 cycles per
+// warp and k step at CPW = 26; the 3x3 layers of a 720 x 480 pair take about
+// 140, a tenth of it for the copies.  All FP32 convolutions of that pair with
+// its re-match: 33.4 ms in k_conv_nt (14 warps per SM on four schedulers, 8
+// pack moves per 32 fmas, a row's last tile), now 22.5; of a KITTI pair in 2x2
+// layers 14.5 and 9.7 ms; of a 256 x 192 grey pair 4.58 and 2.55 ms.  Of that
+// the order of the fmas and the operands loaded a step ahead gave 4 % and
+// tanh_pair 7 to 15 %.  Measured and left out: three CTAs at 160 to 168
+// registers (23.0 to 23.2 ms), scalar fmas, exactly 25 channels per warp with
+// one unpaired (2 % slower).
 constexpr int PXT = 128, PXS = 3, PXP = 20; // pixels per CTA, slices in flight, floats of a pixel's slice
-__host__ __device__ constexpr int cpw_pitch(int CPW) { return (CPW + 3) / 4 * 4; } // floats of a warp's weights per k
+// a k row of weights in shared memory: warp w's channels are wmain = CPW / 4 * 4 from wmain w on and, where CPW is not a
+// multiple of 4, the pair from 4 wmain + 2 w on: 16- and 8-byte loads out of rows copied as they lie in memory
+__host__ __device__ constexpr int w_main(int CPW) { return CPW / 4 * 4; }
+__host__ __device__ constexpr int w_pitch(int CPW) { return CPW > 16 ? BN : 64; }
 __host__ __device__ constexpr int epi_pitch(int CPW) { return CPW / 2 % 2 ? CPW : CPW + 2; } // floats of a pixel in the epilogue
-__host__ __device__ constexpr int px_stage(int CPW, int TK) { return PXT * PXP + TK * 4 * cpw_pitch(CPW); }
+__host__ __device__ constexpr int px_stage(int CPW, int TK) { return PXT * PXP + TK * w_pitch(CPW); }
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src)
 {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async8(uint32_t dst, const void *src)
+// shared-memory loads that stay where they are written in the k loop
+__device__ __forceinline__ void lds_f4(const float *p, float (&v)[4])
 {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void lds_u2(const float *p, unsigned long long &a, unsigned long long &b)
+{
+    asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"((uint32_t)__cvta_generic_to_shared(p)));
 }
 
-// accumulators of 4 pixels x CPW / 2 channel pairs; four (or kn) k steps on them: A the lane's pixel, B the warp's weights
+// accumulators of 4 pixels x CPW / 2 channel pairs, and k steps on them: A the lane's pixel, B the warp's run of weights,
+// Bt the pair beyond it
 template <int CPW> struct PxAcc {
     unsigned long long v[4][CPW / 2];
     __device__ __forceinline__ PxAcc()
@@ -343,24 +356,61 @@ template <int CPW> struct PxAcc {
 #pragma unroll
             for (int m = 0; m < CPW / 2; ++m) v[i][m] = 0ull;
     }
-    // ap: the pixels' input of this k, duplicated
-    __device__ __forceinline__ void step(const unsigned long long (&ap)[4], const float *b)
+    // ap: the pixels' input of this k, duplicated.  The pixel index snakes, so that every fma shares an operand register
+    // with the one before it
+    __device__ __forceinline__ void step(const unsigned long long (&ap)[4], const float *b, const float *bt)
     {
+        unsigned long long bv[CPW / 2];
 #pragma unroll
         for (int m = 0; m + 1 < CPW / 2; m += 2) {
-            const ulonglong2 bv = *(const ulonglong2 *)(b + 2 * m);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) fma2(v[i][m], ap[i], bv.x), fma2(v[i][m + 1], ap[i], bv.y);
+            const ulonglong2 t = *(const ulonglong2 *)(b + 2 * m);
+            bv[m] = t.x, bv[m + 1] = t.y;
         }
-        if (CPW / 2 % 2) {
-            const unsigned long long bv = *(const unsigned long long *)(b + CPW - 2);
+        if (CPW / 2 % 2) bv[CPW / 2 - 1] = *(const unsigned long long *)bt;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) fma2(v[i][CPW / 2 - 1], ap[i], bv);
+        for (int m = 0; m < CPW / 2; ++m)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int i = m % 2 ? 3 - j : j;
+                fma2(v[i][m], ap[i], bv[m]);
+            }
+    }
+    // NK k steps, the operands of a step loaded during the one before it
+    template <int PITCH, int NK> __device__ __forceinline__ void slice(const float *A, const float *B, const float *Bt)
+    {
+        constexpr int WB = w_pitch(CPW), M = CPW / 2;
+        float av[2][4][4];
+        unsigned long long bv[2][M];
+        auto loadA = [&](int q) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) lds_f4(A + 32 * PITCH * i + 4 * q, av[q & 1][i]);
+        };
+        auto loadB = [&](int k) {
+#pragma unroll
+            for (int m = 0; m + 1 < M; m += 2) lds_u2(B + k * WB + 2 * m, bv[k & 1][m], bv[k & 1][m + 1]);
+            if (M % 2) bv[k & 1][M - 1] = *(const unsigned long long *)(Bt + k * WB);
+        };
+        loadA(0);
+        loadB(0);
+#pragma unroll
+        for (int k = 0; k < NK; ++k) {
+            if (k + 1 < NK) loadB(k + 1);
+            if (k % 4 == 1 && k / 4 + 1 < NK / 4) loadA(k / 4 + 1);
+            unsigned long long ap[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) ap[i] = pack2(av[k / 4 & 1][i][k % 4], av[k / 4 & 1][i][k % 4]);
+#pragma unroll
+            for (int m = 0; m < M; ++m)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int i = m % 2 ? 3 - j : j;
+                    fma2(v[i][m], ap[i], bv[k & 1][m]);
+                }
         }
     }
-    template <int PITCH> __device__ __forceinline__ void steps(const float *A, const float *B, int kn = 4)
+    template <int PITCH> __device__ __forceinline__ void steps(const float *A, const float *B, const float *Bt, int kn = 4)
     {
-        constexpr int WB = 4 * cpw_pitch(CPW);
+        constexpr int WB = w_pitch(CPW);
         float av[4][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -373,10 +423,77 @@ template <int CPW> struct PxAcc {
             unsigned long long ap[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) ap[i] = pack2(av[i][k], av[i][k]);
-            step(ap, B + k * WB);
+            step(ap, B + k * WB, Bt + k * WB);
         }
     }
 };
+
+__device__ __forceinline__ void unpack2(unsigned long long v, float &lo, float &hi)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long vfma2(unsigned long long a, unsigned long long b, unsigned long long c)
+{
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ unsigned long long vadd2(unsigned long long a, unsigned long long b)
+{
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long vmul2(unsigned long long a, unsigned long long b)
+{
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
+// cnncrf_tanhf of two values, the same bits, without branches and on packed operations where it has two of them:
+//   rint of 0 <= y < 2^22 is (y + 1.5 2^23) - 1.5 2^23, and the sum's low bits are the integer;
+//   2 |x| <= 18 needs no range case of expm1, 2^0 em1 + (2^0 - 1) is em1, and the quotient at |x| = 9 rounds to 1;
+//   the quotient E / (E + 2) by Markstein's correctly rounded division ("Computation of elementary functions on the
+//   IBM RISC System/6000 processor", 1990): a reciprocal y refined by one Newton step, q = E y, q + y (E - q (E + 2)).
+//   Its operands are those of the 2^27 or so floats between 2^-12 and 9, and each was compared with cnncrf_tanhf.
+__device__ __forceinline__ float2 tanh_pair(float2 x)
+{
+    auto both = [](float c) { return pack2(c, c); };
+    float ax, ay; // |x|, at most 9; NaN stays
+    asm("min.NaN.f32 %0, %1, 0f41100000;" : "=f"(ax) : "f"(fabsf(x.x)));
+    asm("min.NaN.f32 %0, %1, 0f41100000;" : "=f"(ay) : "f"(fabsf(x.y)));
+    const unsigned long long a = pack2(ax, ay), v = vadd2(a, a);
+    const unsigned long long z = vadd2(vmul2(v, both(CNNCRF_INV_LN2)), both(12582912.0f));
+    const unsigned long long n = vadd2(z, both(-12582912.0f));
+    unsigned long long r = vfma2(n, both(-CNNCRF_LN2_HI), v);
+    r = vfma2(n, both(-CNNCRF_LN2_LO), r);
+    float zx, zy;
+    unpack2(z, zx, zy);
+    const unsigned long long s = pack2(__int_as_float((__float_as_int(zx) << 23) + 0x3f800000),
+                                       __int_as_float((__float_as_int(zy) << 23) + 0x3f800000)); // 2^n
+    unsigned long long q = vfma2(both(CNNCRF_C8), r, both(CNNCRF_C7));
+    q = vfma2(q, r, both(CNNCRF_C6));
+    q = vfma2(q, r, both(CNNCRF_C5));
+    q = vfma2(q, r, both(CNNCRF_C4));
+    q = vfma2(q, r, both(CNNCRF_C3));
+    q = vfma2(q, r, both(CNNCRF_C2));
+    const unsigned long long em1 = vfma2(vmul2(r, r), q, r);
+    const unsigned long long e = vfma2(s, em1, vadd2(s, both(-1.0f)));
+    const unsigned long long d = vadd2(e, both(2.0f)), nd = vfma2(e, both(-1.0f), both(-2.0f));
+    float dx, dy, yx, yy;
+    unpack2(d, dx, dy);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yx) : "f"(dx));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(yy) : "f"(dy));
+    unsigned long long y = pack2(yx, yy);
+    y = vfma2(vfma2(nd, y, both(1.0f)), y, y);
+    const unsigned long long t0 = vmul2(e, y), t = vfma2(vfma2(nd, t0, e), y, t0);
+    float tx, ty;
+    unpack2(t, tx, ty);
+    tx = ax < 2.44140625e-4f ? x.x : copysignf(tx, x.x);
+    ty = ay < 2.44140625e-4f ? x.y : copysignf(ty, x.y);
+    return make_float2(tx, ty);
+}
 
 // The warp's 128 pixels x CPW channels through shared memory, then a rolled loop of bias, activation and store on
 // channel pairs, a pixel's channels as one run (unrolled on the registers, the activations were 66 KB of code that
@@ -386,36 +503,53 @@ __device__ __forceinline__ void px_epilogue(const ConvArgs &a, const PxAcc<CPW> 
                                             int Wo, int lane, int warp)
 {
     constexpr int EP = epi_pitch(CPW);
+    constexpr int NM = w_main(CPW) / 2, NP = CPW / 2; // channel pairs of the warp's run, and with the one beyond it
     float *st = sm + warp * PXT * EP;
-    const int c0 = warp * CPW, nc = min(CPW, a.Cout - c0);
-    if (nc <= 0) return;
+    const int c0 = warp * w_main(CPW), ct = 4 * w_main(CPW) + 2 * warp;
+    if (c0 >= a.Cout) return;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int m = 0; m < CPW / 2; ++m) *(unsigned long long *)(st + (lane + 32 * i) * EP + 2 * m) = acc.v[i][m];
+        for (int m = 0; m < NP; ++m) *(unsigned long long *)(st + (lane + 32 * i) * EP + 2 * m) = acc.v[i][m];
     __syncwarp();
     const bool dense = a.out_ch == 1 && a.out_row == Wo * a.out_pix;
-    const bool pairs = dense && a.out_pix % 2 == 0 && nc % 2 == 0 && ((uintptr_t)outp & 7) == 0;
-    const int np = (nc + 1) / 2, dq = 32 / np, dm = 32 - dq * np; // channel pairs; a lane's stride in pixels and pairs
-    int q = lane / np, m = lane - q * np;
+    const bool pairs = dense && a.out_pix % 2 == 0 && ((uintptr_t)outp & 7) == 0;
+    constexpr int DQ = 32 / NP, DM = 32 - DQ * NP; // a lane's stride in pixels and pairs
+    int q = lane / NP, m = lane - q * NP;
+    constexpr int U = 4; // pairs of a lane at a time
+    static_assert(PXT * NP % (32 * U) == 0, "px_epilogue rounds");
 #pragma unroll 1
-    for (int e = lane; e < PXT * np; e += 32) {
-        const int c = 2 * m, p = p0 + q;
-        if (p < npx) {
-            float2 t = *(const float2 *)(st + q * EP + c);
-            if (a.bias) t.x = __fadd_rn(t.x, __ldg(a.bias + c0 + c)), t.y = __fadd_rn(t.y, __ldg(a.bias + c0 + c + 1));
-            t.x = act_fn(t.x, a.act), t.y = act_fn(t.y, a.act);
-            if (pairs) {
-                *(float2 *)(outp + (long)p * a.out_pix + c0 + c) = t;
+    for (int e = 0; e < PXT * NP / 32; e += U) {
+        float2 t[U];
+        int pp[U], cc[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            pp[u] = p0 + q, cc[u] = m < NM ? c0 + 2 * m : ct;
+            t[u] = *(const float2 *)(st + q * EP + 2 * m);
+            if (a.bias) t[u].x = __fadd_rn(t[u].x, __ldg(a.bias + cc[u])), t[u].y = __fadd_rn(t[u].y, __ldg(a.bias + cc[u] + 1));
+            m += DM, q += DQ;
+            if (m >= NP) m -= NP, ++q;
+        }
+        if (a.act & 1)
+#pragma unroll
+            for (int u = 0; u < U; ++u) t[u] = tanh_pair(t[u]);
+        if (a.act & 2)
+#pragma unroll
+            for (int u = 0; u < U; ++u) t[u].x = fabsf(t[u].x), t[u].y = fabsf(t[u].y);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int p = pp[u], c = cc[u];
+            if (p >= npx || c >= a.Cout) continue;
+            const bool both = c + 1 < a.Cout;
+            if (pairs && both) {
+                *(float2 *)(outp + (long)p * a.out_pix + c) = t[u];
             } else {
                 const int y = dense ? 0 : p / Wo, x = p - y * Wo;
-                float *o = outp + (long)y * a.out_row + (long)x * a.out_pix + (long)(c0 + c) * a.out_ch;
-                o[0] = t.x;
-                if (c + 1 < nc) o[a.out_ch] = t.y;
+                float *o = outp + (long)y * a.out_row + (long)x * a.out_pix + (long)c * a.out_ch;
+                o[0] = t[u].x;
+                if (both) o[a.out_ch] = t[u].y;
             }
         }
-        m += dm, q += dq;
-        if (m >= np) m -= np, ++q;
     }
 }
 
@@ -423,8 +557,7 @@ template <int CPW, int TK>
 __global__ void __launch_bounds__(128, 2) k_conv_px(ConvArgs a, int npx, int Wo, int K)
 {
     constexpr int NQ = TK / 4;         // 16-byte pieces of a pixel's slice
-    constexpr int PP = cpw_pitch(CPW); // a warp's weights per k
-    constexpr int WB = 4 * PP;         // a k row of weights
+    constexpr int WB = w_pitch(CPW);   // a k row of weights
     constexpr int SF = px_stage(CPW, TK);
     static_assert(CPW % 2 == 0 && TK % 4 == 0 && TK <= PXP && 4 * CPW <= BN, "k_conv_px tile");
     extern __shared__ float4 sm4[];
@@ -454,18 +587,11 @@ __global__ void __launch_bounds__(128, 2) k_conv_px(ConvArgs a, int npx, int Wo,
             const uint32_t o = 4u * SF * lbuf;
 #pragma unroll
             for (int j = 0; j < NQ; ++j) cp_async16(pdst[j] + o, src + poff[j]);
-            constexpr int CF = CPW % 4 == 0 ? 4 : 2, NC = CPW / CF; // floats of a copy, copies per warp and k
-            const uint32_t d = sm_s + o + 4 * PXT * PXP;
+            const uint32_t d = sm_s + o + 4 * PXT * PXP + 16 * tid;
 #pragma unroll
-            for (int f0 = 0; f0 < TK * 4 * NC; f0 += 128) {
-                const int f = f0 + tid;
-                if (f < TK * 4 * NC) {
-                    const int k = f / (4 * NC), r = f - k * (4 * NC), g = r / NC, c = r - g * NC;
-                    const uint32_t dst = d + (k * WB + g * PP + c * CF) * 4;
-                    if (CF == 4) cp_async16(dst, wsrc + k * BN + g * CPW + c * CF);
-                    else cp_async8(dst, wsrc + k * BN + g * CPW + c * CF);
-                }
-            }
+            for (int f = 0; f < TK * WB / 4; f += 128)
+                if (f + 128 <= TK * WB / 4 || f + tid < TK * WB / 4)
+                    cp_async16(d + 16 * f, WB == BN ? wsrc + 4 * (f + tid) : wsrc + (f + tid) / (WB / 4) * BN + (f + tid) % (WB / 4) * 4);
             wsrc += TK * BN;
             ci += TK, src += TK;
             if (ci == a.Cin) {
@@ -483,9 +609,9 @@ __global__ void __launch_bounds__(128, 2) k_conv_px(ConvArgs a, int npx, int Wo,
         asm volatile("cp.async.wait_group %0;" ::"n"(PXS - 2) : "memory");
         __syncthreads(); // slice s is there; everyone is done with slice s - 1
         load();
-        const float *A = sm + cur * SF + lane * PXP, *B = sm + cur * SF + PXT * PXP + warp * PP;
-#pragma unroll
-        for (int q = 0; q < NQ; ++q, A += 4, B += 4 * WB) acc.template steps<PXP>(A, B);
+        const float *A = sm + cur * SF + lane * PXP, *B = sm + cur * SF + PXT * PXP + warp * w_main(CPW);
+        const float *Bt = sm + cur * SF + PXT * PXP + 4 * w_main(CPW) + 2 * warp;
+        acc.template slice<PXP, TK>(A, B, Bt);
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
@@ -497,11 +623,11 @@ __global__ void __launch_bounds__(128, 2) k_conv_px(ConvArgs a, int npx, int Wo,
 // pitch, and all K rows of the weights in shared memory.  Bound by the tanh
 // epilogue and the output's bytes; a thread per pixel with all channels in
 // registers stored 4 bytes at a 400-byte stride and took 1.42 ms for a KITTI
-// pair's three first layers, this 0.76.
+// pair's three first layers, this 0.41 (0.75 with cnncrf_tanhf as it stands).
 template <int CPW, int KP>
 __global__ void __launch_bounds__(128, 3) k_conv_patch(ConvArgs a, int npx, int Wo, int K)
 {
-    constexpr int PP = cpw_pitch(CPW), WB = 4 * PP;
+    constexpr int WB = w_pitch(CPW);
     static_assert(KP % 8 == 4, "conflict-free pixel pitch");
     extern __shared__ float4 sm4[];
     float *A = (float *)sm4, *B = A + PXT * KP; // [PXT][KP], [K][WB]
@@ -516,15 +642,15 @@ __global__ void __launch_bounds__(128, 3) k_conv_patch(ConvArgs a, int npx, int 
             for (int kx = 0; kx < a.kw; ++kx)
                 for (int ci = 0; ci < a.Cin; ++ci) *d++ = __ldg(src + (long)ky * a.in_row + (long)kx * a.in_pix + ci);
     }
-    for (int i = tid; i < K * 4 * CPW; i += 128) {
-        const int k = i / (4 * CPW), c = i - k * (4 * CPW), g = c / CPW;
-        B[k * WB + g * PP + c - g * CPW] = __ldg(a.wt + (long)k * BN + c);
+    for (int i = tid; i < K * CPW; i += 128) {
+        const int k = i / CPW, c = i - k * CPW;
+        *(float4 *)(B + k * WB + 4 * c) = __ldg((const float4 *)(a.wt + (long)k * BN + 4 * c));
     }
     __syncthreads();
     PxAcc<CPW> acc;
-    const float *Ap = A + lane * KP, *Bp = B + warp * PP;
+    const float *Ap = A + lane * KP, *Bp = B + warp * w_main(CPW), *Bt = B + 4 * w_main(CPW) + 2 * warp;
 #pragma unroll 1
-    for (int k = 0; k < K; k += 4, Ap += 4, Bp += 4 * WB) acc.template steps<KP>(Ap, Bp, K - k);
+    for (int k = 0; k < K; k += 4, Ap += 4, Bp += 4 * WB, Bt += 4 * WB) acc.template steps<KP>(Ap, Bp, Bt, K - k);
     __syncthreads();
     px_epilogue<CPW>(a, acc, A, outp, p0, npx, Wo, lane, warp);
 }
@@ -540,7 +666,7 @@ template <int CPW, int TK> int launch_px(const ConvArgs &a, int Ho, int Wo, int 
 
 template <int CPW, int KP> int launch_patch(const ConvArgs &a, int Ho, int Wo, int K, cudaStream_t st)
 {
-    const int sm = 4 * std::max(PXT * KP + K * 4 * cpw_pitch(CPW), 4 * PXT * epi_pitch(CPW));
+    const int sm = 4 * std::max(PXT * KP + K * w_pitch(CPW), 4 * PXT * epi_pitch(CPW));
     CNNCRF_CUDA(cudaFuncSetAttribute(k_conv_patch<CPW, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
     CNNCRF_PROF("conv_first", st);
     k_conv_patch<CPW, KP><<<dim3(ceil_div((long)Ho * Wo, PXT), a.n_img), 128, sm, st>>>(a, Ho * Wo, Wo, K);

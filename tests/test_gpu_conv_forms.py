@@ -38,3 +38,38 @@ def test_net_bitexact_over_kernels(cuda, oracle, topology, ic, feat, pw, W, H):
     ovol, opw = oracle.predict(cfg, params, lp, rp, oracle.disparity_list(0.0, float(D - 1), 1.0))
     assert np.array_equal(vol.cpu().numpy(), ovol)
     assert np.array_equal(net.pairwise_out.cpu().numpy(), opw)
+
+
+def test_epilogue_tanh_bitexact(cuda, oracle):
+    """The epilogue's tanh of value pairs equals the oracle's, bit for bit: as
+    the biases of layers with zero weights, in the first-layer kernel (one
+    layer) and the wide one (two), values around every case of the function
+    (2^-12, 9, the exponents' reductions, zeros, infinities, denormals)."""
+    torch = cuda
+    from cnncrf.api import StereoNet
+    f = np.float32
+    x = [0.0, -0.0, np.inf, -np.inf, 1e-45, -1e-40, 1e-30, 3e38, -3e38, 88.0, 20.0]
+    for c in [2.0 ** -12, 9.0, 1.0, 8.9999] + [0.25 * np.log(2.0) * (2 * k + 1) for k in range(28)]:
+        v = f(c)
+        for _ in range(4):
+            v = np.nextafter(v, f(0))
+        for _ in range(9):
+            x += [v, -v]
+            v = np.nextafter(v, f(100))
+    x = np.concatenate([np.array(x, f), np.random.default_rng(3).uniform(-10, 10, 3000).astype(f)])
+    x = np.resize(x, (x.size + 99) // 100 * 100).reshape(-1, 100)
+    ref = oracle.conv(x.reshape(1, -1, 1), np.ones((1, 1, 1, 1), f), None, act=1).reshape(x.shape)
+    for layers in (1, 2):
+        h = 3 if layers == 1 else 5
+        net = StereoNet(layers, 1, 3, h, h, topology=1)
+        net.init_net(0.0, 0.0, 1.0)
+        for i in range(net.num_params()):
+            net.set_param(i, np.zeros(net.param_shape(i), f))
+        im = torch.rand((h, h, 4), device="cuda")
+        for row, want in zip(x, ref):
+            net.set_param(2 * layers - 1, row)
+            net.predict(im, im)
+            for side in (0, 1):
+                got = net.features(side).cpu().numpy()[0, 0]
+                assert np.array_equal(got.view(np.int32) & 0x7fffffff, want.view(np.int32) & 0x7fffffff)
+                assert np.array_equal(got, want)
