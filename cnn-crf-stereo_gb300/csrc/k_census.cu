@@ -228,7 +228,8 @@ __global__ void k_quadfit_direct(float *__restrict__ u, const float *__restrict_
 // The same on the solver's own arrays: its C1 is theta - phi, of which a pixel reads three values; writing out all D of
 // them first took 139 us of a 720 x 480 pair at 128 labels, this kernel takes about as long as the fit on a given C1 (16 us).
 __global__ void k_quadfit_solver(float *__restrict__ u, const float *__restrict__ cost, const uint16_t *__restrict__ costq,
-                                 float qs, float qo, const float *__restrict__ phi, long npx, int D, float dmin, float dstep)
+                                 float qs, float qo, const float *__restrict__ phi, int DP, long npx, int D, float dmin,
+                                 float dstep)
 {
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= npx) return;
@@ -236,7 +237,7 @@ __global__ void k_quadfit_solver(float *__restrict__ u, const float *__restrict_
     if (z <= 0 || z >= D - 1) return;
     auto c = [&](int k) {
         const long o = i * D + k;
-        return __fsub_rn(costq ? __fmaf_rn((float)costq[o], qs, qo) : cost[o], phi[o]);
+        return __fsub_rn(costq ? __fmaf_rn((float)costq[o], qs, qo) : cost[o], phi[i * DP + k]);
     };
     u[i] = quadfit(u[i], c(z - 1), c(z), c(z + 1), dstep);
 }
@@ -339,12 +340,12 @@ int quadfit_direct(float *u, const float *c1, long npx, int D, float dmin, float
     return CNNCRF_OK;
 }
 
-int quadfit_solver(float *u, const float *cost, const void *costq, UnaryQ16 q, const float *phi, long npx, int D, float dmin,
+int quadfit_solver(float *u, const float *cost, const void *costq, UnaryQ16 q, const float *phi, int DP, long npx, int D, float dmin,
                    float dstep, cudaStream_t st)
 {
     {
         CNNCRF_PROF("quadfit", st);
-        k_quadfit_solver<<<ceil_div(npx, 256), 256, 0, st>>>(u, cost, (const uint16_t *)costq, q.scale, q.offset, phi, npx, D,
+        k_quadfit_solver<<<ceil_div(npx, 256), 256, 0, st>>>(u, cost, (const uint16_t *)costq, q.scale, q.offset, phi, DP, npx, D,
                                                              dmin, dstep);
     }
     CNNCRF_CHECK_LAUNCH();

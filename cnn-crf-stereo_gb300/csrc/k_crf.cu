@@ -71,14 +71,15 @@ __global__ void k_wta(const float *__restrict__ cost, long npx, int D, int32_t *
 }
 
 __global__ void k_c1(const float *__restrict__ cost, const uint16_t *__restrict__ costq, float qs, float qo,
-                     const float *__restrict__ phi, long n, float *__restrict__ out)
+                     const float *__restrict__ phi, long n, int D, int DP, float *__restrict__ out)
 {
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = __fsub_rn(costq ? __fmaf_rn((float)costq[i], qs, qo) : cost[i], phi[i]);
+    if (i < n) out[i] = __fsub_rn(costq ? __fmaf_rn((float)costq[i], qs, qo) : cost[i], phi[i / D * DP + i % D]);
 }
 
 struct Layout {
     size_t phi, lbuf, ch, cv, lb, total;
+    int pitch; // labels from one vector of phi and lbuf to the next
 };
 
 Layout layout(int W, int H, int D, int np = 1)
@@ -92,6 +93,13 @@ Layout layout(int W, int H, int D, int np = 1)
     l.cv = al(l.ch + (size_t)H * np * sizeof(double));
     l.lb = al(l.cv + (size_t)W * np * sizeof(double));
     l.total = al(l.lb + np * sizeof(double));
+    // The two arrays of N D floats hold phi at a pitch of whole 16-byte chunks where the messages, one per block of
+    // BLK nodes, leave the room for it: from 3 labels on unless the image is a few pixels wide or high
+    l.pitch = (D + 3) / 4 * 4;
+    const size_t blocks = std::max((size_t)H * ((W + BLK - 1) / BLK), (size_t)W * ((H + BLK - 1) / BLK));
+    const size_t lbuf = al((size_t)W * H * np * l.pitch * sizeof(float));
+    if (lbuf + blocks * np * l.pitch * sizeof(float) <= l.ch) l.lbuf = lbuf;
+    else l.pitch = D;
     return l;
 }
 
@@ -102,9 +110,9 @@ int lane_labels(int D)
     return P <= 2 ? P : (P <= 4 ? 4 : (P <= 6 ? 6 : 8));
 }
 
-size_t form_smem(int D, bool hpass, bool t16, const CrfForm &f)
+size_t form_smem(int D, bool hpass, bool t16, int mode, const CrfForm &f)
 {
-    return sizeof(float) * (f.paired ? 1 : f.wpb) * (size_t)chain_floats(lane_labels(D), hpass, t16, D % 4 != 0, f.paired, f.buffers);
+    return sizeof(float) * (f.paired ? 1 : f.wpb) * (size_t)chain_floats(lane_labels(D), hpass, t16, mode, f.paired, f.buffers);
 }
 
 // How a pass runs on this GPU's 152 SMs.
@@ -126,7 +134,7 @@ CrfForm choose_form(const CrfPassArgs &a, bool hpass, int ring, int wpb)
     const long chains = (long)(hpass ? a.H : a.W) * a.np;
     auto resident = [&](const CrfForm &f) {
         const long ctas = (chains + (f.paired ? 1 : f.wpb) - 1) / (f.paired ? 1 : f.wpb);
-        return (long)(form_smem(a.D, hpass, t16, f) + SMEM_CTA) * ((ctas + SMS - 1) / SMS) <= SMEM_SM;
+        return (long)(form_smem(a.D, hpass, t16, vec_mode(a, hpass), f) + SMEM_CTA) * ((ctas + SMS - 1) / SMS) <= SMEM_SM;
     };
     CrfForm f{true, 2, wpb};
     f.paired = chains <= 8 * SMS && resident(f);
@@ -149,10 +157,10 @@ int pass(const CrfPassArgs &a, bool hpass, int delta, int ring, int wpb, cudaStr
     }
 }
 
-// whether a CTA of the smallest form fits (it does for every label count and wpb; an upper bound for the 16-bit unary)
+// whether a CTA of the smallest form fits (it does for every label count and wpb; an upper bound for the other vector modes)
 bool fits(int D, bool hpass, int wpb)
 {
-    return form_smem(D, hpass, false, CrfForm{false, 2, wpb}) <= 227 * 1024;
+    return form_smem(D, hpass, false, RAGGED, CrfForm{false, 2, wpb}) <= 227 * 1024;
 }
 
 // the tile of the tuning table for this shape, each pass falling back to the
@@ -177,7 +185,7 @@ CrfPassArgs pass_args(const float *cost, long wps, int W, int H, int D, int np, 
     a.qoffset23 = q.offset - 8388608.0f * q.scale;
     a.phi = (float *)(ws + l.phi);
     a.lbuf = (float *)(ws + l.lbuf);
-    a.W = W, a.H = H, a.D = D, a.np = np, a.wps = wps;
+    a.W = W, a.H = H, a.D = D, a.DP = l.pitch, a.np = np, a.wps = wps;
     a.rp = rp;
     a.store_phi = 1;
     return a;
@@ -367,23 +375,25 @@ const double *crf_lb_device(const void *ws, int W, int H, int D, int npairs)
     return (const double *)((const char *)ws + layout(W, H, D, npairs).lb);
 }
 
-int crf_c1(const float *cost, const void *ws, long n, float *out, cudaStream_t st, int D, const void *costq,
+int crf_c1(const float *cost, const void *ws, int W, int H, int D, float *out, cudaStream_t st, const void *costq,
            UnaryQ16 q)
 {
+    const long n = (long)W * H * D;
     const float *phi = (const float *)ws;
     const uint16_t *cq = (costq && crf_reads_q16(D)) ? (const uint16_t *)costq : nullptr;
     {
         CNNCRF_PROF("c1", st);
-        k_c1<<<ceil_div(n, 256), 256, 0, st>>>(cost, cq, q.scale, q.offset, phi, n, out);
+        k_c1<<<ceil_div(n, 256), 256, 0, st>>>(cost, cq, q.scale, q.offset, phi, n, D, layout(W, H, D).pitch, out);
     }
     CNNCRF_CHECK_LAUNCH();
     return CNNCRF_OK;
 }
 
-int crf_quadfit(float *u, const float *cost, const void *ws, long npx, int D, float dmin, float dstep, cudaStream_t st,
+int crf_quadfit(float *u, const float *cost, const void *ws, int W, int H, int D, float dmin, float dstep, cudaStream_t st,
                 const void *costq, UnaryQ16 q)
 {
-    return quadfit_solver(u, cost, costq && crf_reads_q16(D) ? costq : nullptr, q, (const float *)ws, npx, D, dmin, dstep, st);
+    return quadfit_solver(u, cost, costq && crf_reads_q16(D) ? costq : nullptr, q, (const float *)ws, layout(W, H, D).pitch,
+                          (long)W * H, D, dmin, dstep, st);
 }
 
 } // namespace k

@@ -28,10 +28,11 @@ struct CrfPassArgs {
     const uint16_t *thetaq; // its 16-bit fixed-point copy, read by the H pass instead of theta when set
     float qscale, qoffset;  // theta = q * qscale + qoffset (exact in FP32)
     float qoffset23;        // qoffset - 2^23 qscale, exact: theta = (2^23 + q) * qscale + qoffset23
-    float *phi;         // H/V split of the unary, same layout
+    float *phi;         // H/V split of the unary [np][H][W][DP]
     const float *wgt;   // wx (H pass) or wy (V pass), pair stride wps
-    float *lbuf;        // forward messages, same layout as phi
+    float *lbuf;        // each block's first forward message, [np][H][blocks][DP] in an H pass, [np][blocks][W][DP] in a V pass
     int W, H, D, np;
+    int DP;              // labels from one vector of phi and lbuf to the next: D rounded up to 4, or D (crf_pitch)
     long wps;
     Rho rp;
     int first;           // H pass of the first iteration: phi = 0, not read
@@ -56,23 +57,31 @@ int crf_pass_p4(const CrfPassArgs &a, bool hpass, int delta, const CrfForm &f, c
 int crf_pass_p6(const CrfPassArgs &a, bool hpass, int delta, const CrfForm &f, cudaStream_t st);
 int crf_pass_p8(const CrfPassArgs &a, bool hpass, int delta, const CrfForm &f, cudaStream_t st);
 
+// how a pass's vectors lie in memory: on 16 bytes throughout; the cost volume's on any float and phi's on 16 bytes (an H
+// pass whose D is no multiple of 4); both on any float
+enum : int { ALIGNED = 0, SPREAD = 1, RAGGED = 2 };
+inline int vec_mode(const CrfPassArgs &a, bool hpass)
+{
+    return a.D % 4 == 0 ? ALIGNED : (a.DP % 4 ? RAGGED : (hpass ? SPREAD : ALIGNED));
+}
+
 // a chain's shared memory in floats: per block buffer two planes of BLK node vectors, the unary (H pass; 16-bit codes
 // take half the floats) and phi (RAGGED vectors carry up to 3 floats of their neighbours at either end); one block of
 // messages and of edge costs, or two with paired warps
-__host__ __device__ constexpr int vec_floats(int P, bool ragged) { return 32 * P + (ragged ? 4 : 0); }
-__host__ __device__ constexpr int theta_floats(int P, bool hpass, bool t16, bool ragged)
+__host__ __device__ constexpr int vec_floats(int P, int mode) { return 32 * P + (mode == RAGGED ? 4 : 0); }
+__host__ __device__ constexpr int theta_floats(int P, bool hpass, bool t16, int mode)
 {
-    return hpass ? (t16 ? 16 * P : vec_floats(P, ragged)) : 0;
+    return hpass ? BLK * (t16 ? 16 * P : vec_floats(P, mode)) : 0;
 }
-__host__ __device__ constexpr int block_floats(int P, bool hpass, bool t16, bool ragged)
+__host__ __device__ constexpr int block_floats(int P, bool hpass, bool t16, int mode)
 {
-    return BLK * (theta_floats(P, hpass, t16, ragged) + vec_floats(P, ragged));
+    return theta_floats(P, hpass, t16, mode) + BLK * vec_floats(P, mode);
 }
 constexpr int EDGE = 8;                // EDGE: floats of an edge's costs (w rho_1 .. w rho_4, w L2)
 constexpr int EDGES = (BLK + 1) * EDGE;       // of the edges a block uses
-__host__ __device__ constexpr int chain_floats(int P, bool hpass, bool t16, bool ragged, bool paired, int buffers)
+__host__ __device__ constexpr int chain_floats(int P, bool hpass, bool t16, int mode, bool paired, int buffers)
 {
-    return buffers * block_floats(P, hpass, t16, ragged) + (paired ? 2 : 1) * (BLK * 32 * P + EDGES);
+    return buffers * block_floats(P, hpass, t16, mode) + (paired ? 2 : 1) * (BLK * 32 * P + EDGES);
 }
 
 namespace {
@@ -243,6 +252,10 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, int by
 {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 // all but the newest `left` groups (0..2) are complete
@@ -311,7 +324,26 @@ template <int P> __device__ __forceinline__ void copy_ragged(uint32_t dst, const
 #pragma unroll
         for (int c = 0; c < 8 * P + 1; c += 32)
             if (4 * (lane + c) < D + mis) cp_async16(d + 16 * c, base + c0 + 4 * c, 4 * (int)min(4L, total - c0 - 4 * c));
-        o += ns, d += 4 * vec_floats(P, true);
+        o += ns, d += 4 * vec_floats(P, RAGGED);
+    };
+    if (cnt == BLK) {
+#pragma unroll
+        for (int j = 0; j < BLK; ++j) node();
+    } else {
+        for (int j = 0; j < cnt; ++j) node();
+    }
+}
+
+// `cnt` vectors of any D labels that lie one after the other, into slots of 32 P labels, float by float
+template <int P> __device__ __forceinline__ void copy_spread(uint32_t dst, const float *src, int lane, int cnt, int D)
+{
+    const float *g = src + lane;
+    uint32_t d = dst + 4 * lane;
+    auto node = [&]() {
+#pragma unroll
+        for (int c = 0; c < P; ++c)
+            if (lane + 32 * c < D) cp_async4(d + 128 * c, g + 32 * c);
+        g += D, d += 128 * P;
     };
     if (cnt == BLK) {
 #pragma unroll
@@ -432,9 +464,20 @@ template <int P, bool ALIGNED> __device__ __forceinline__ void load_vec(const fl
 // A chain is walked in blocks of BLK nodes.  The block's pixel vectors come
 // from a ring of block buffers in shared memory, filled `buffers` - 1 blocks
 // ahead, so that the chain's dependent arithmetic does not wait on DRAM:
-//   !RAGGED  D a multiple of 4: 16-byte cp.async by the whole warp, several
-//            nodes per instruction where they are small or contiguous
-//   RAGGED   any D: the 16-byte chunks that hold each vector
+//   ALIGNED     16-byte cp.async by the whole warp, several nodes per
+//               instruction where they are small or contiguous
+//   SPREAD      D not a multiple of 4: phi as above, the volume's vectors
+//               float by float into the same slots
+//   RAGGED      the 16-byte chunks that hold each vector, where the workspace
+//               does not hold phi at a pitch of whole chunks (crf_pitch)
+// Vectors at a pitch DP > D carry pad labels D..DP - 1 along.  The H pass
+// that starts a solve stores them as +inf, a V pass turns that into NaN, and
+// neither ever wins a minimum.  D = 75, of a 619 x 271 solve, against RAGGED
+// vectors (four-way bank conflicts on each, masks, single-float stores): the H
+// pass 196 -> 107 us, the V pass 106 -> 81 us, as D = 76; D = 255 of a KITTI
+// pair 1354 -> 511 and 828 -> 377 us.  Measured and left out: the volume's
+// block as one run of 16-byte copies, each lane shifting its labels into place
+// (150 us) or the copying warp doing so once (155 us).
 // An edge's costs w rho_t and w L2 are multiplied out once per block, an edge
 // per lane, and read back as broadcasts.
 //
@@ -461,7 +504,7 @@ template <int P, bool ALIGNED> __device__ __forceinline__ void load_vec(const fl
 // 34 us).  Measured and left out: bulk copies on mbarriers for the H blocks
 // (a wait costs 150 cycles, cp.async's 43; 338 against 316 us for one pair),
 // and keeping all messages for few chains (276 against 258 us).
-template <int P, int DELTA, bool HPASS, bool T16, bool RAGGED, bool PAIRED>
+template <int P, int DELTA, bool HPASS, bool T16, int MODE, bool PAIRED>
 __global__ void __launch_bounds__(PAIRED ? 64 : 128) k_crf_chain(const CrfPassArgs a, const int NB)
 {
     extern __shared__ float4 smem4[];
@@ -469,41 +512,43 @@ __global__ void __launch_bounds__(PAIRED ? 64 : 128) k_crf_chain(const CrfPassAr
     const bool walks = !PAIRED || warp == 0, helps = !PAIRED || warp == 1; // roles: walk the chain; copy and recompute
     const int wib = PAIRED ? 0 : warp; // the chain within the CTA
     const int gchain = PAIRED ? blockIdx.x : blockIdx.x * (blockDim.x >> 5) + wib;
-    const int W = a.W, H = a.H, D = T16 ? 32 * P : a.D;
+    constexpr bool RAG = MODE == RAGGED, VEC = !RAG; // VEC: phi and lbuf in whole 16-byte chunks
+    const int W = a.W, H = a.H, D = T16 ? 32 * P : a.D, DP = T16 ? 32 * P : (RAG ? a.D : a.DP);
     const int n = HPASS ? W : H;
     const int nch = HPASS ? H : W;
     if (gchain >= nch * a.np) return;
     // pair of the batch and chain within it
     const int pair = gchain / nch, chain = gchain - pair * nch;
     // element offset of the chain's node 0 and the stride between its nodes
-    const long ns = (HPASS ? 1L : (long)W) * D;
-    const long cb = (long)W * H * D * pair + (HPASS ? (long)chain * W : (long)chain) * D;
-    const float *theta = a.theta + cb;
-    const uint16_t *thetaq = T16 ? a.thetaq + cb : nullptr;
+    const long ns = (HPASS ? 1L : (long)W) * DP;
+    const long cn = (long)W * H * pair + (HPASS ? (long)chain * W : (long)chain);
+    const long cb = cn * DP, tcb = cn * D; // of phi; of theta (H passes: its nodes are D apart)
+    const uint16_t *thetaq = T16 ? a.thetaq + tcb : nullptr;
     float *phi = a.phi + cb;
-    float *lbuf = a.lbuf + cb;
+    const int nblk = (n + BLK - 1) / BLK;
+    const long ls = (HPASS ? 1L : (long)W) * DP; // from a block's first message to the next block's
+    float *lbuf = a.lbuf + (HPASS ? ((long)pair * H + chain) * nblk : (long)pair * nblk * W + chain) * DP;
     const float *wgt = a.wgt + a.wps * pair + (HPASS ? (long)chain * W : (long)chain);
     const long wst = HPASS ? 1 : W; // weight of edge e (node e to e + 1) at wgt[e wst]
 
-    constexpr bool RAG = RAGGED, VEC = !RAG; // VEC: 16-byte aligned vectors of a multiple of 4 labels
-    constexpr int LP = 32 * P, VF = vec_floats(P, RAG), TF = theta_floats(P, HPASS, T16, RAG);
-    constexpr int OP = BLK * TF; // planes of a buffer: the unary at 0, phi at OP
-    constexpr int BF = block_floats(P, HPASS, T16, RAG), MF = BLK * LP + EDGES;
-    float *ring = (float *)smem4 + (size_t)wib * chain_floats(P, HPASS, T16, RAG, PAIRED, NB);
+    constexpr int LP = 32 * P, VF = vec_floats(P, MODE), TF = T16 ? 16 * P : VF; // TF: of a node's unary
+    constexpr int OP = theta_floats(P, HPASS, T16, MODE); // planes of a buffer: the unary at 0, phi at OP
+    constexpr int BF = block_floats(P, HPASS, T16, MODE), MF = BLK * LP + EDGES;
+    float *ring = (float *)smem4 + (size_t)wib * chain_floats(P, HPASS, T16, MODE, PAIRED, NB);
     float *msg = ring + NB * BF; // the block's messages and edge costs (PAIRED: of even and odd blocks of the sweep)
     const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring);
     const bool use_phi = !(HPASS && a.first);
 
-    // Labels D..32 P - 1 are pads at +inf: set once, the copies never write
-    // them (RAGGED slots hold other vectors' labels there, and read_node masks
-    // them).  The first H pass copies no phi: zero.
+    // Labels DP..32 P - 1 (of a SPREAD unary D..) are pads at +inf: set once,
+    // the copies never write them (RAGGED slots hold other vectors' labels
+    // there, and read_node masks them).  The first H pass copies no phi: zero.
     if (helps && (D < LP || !use_phi)) {
         for (int i = lane; i < NB * BLK * VF; i += 32) {
             const int nd = i / VF, k = i - nd * VF, q = nd / BLK, j = nd - q * BLK;
             float *s = ring + q * BF;
-            const bool pad = k >= D;
+            const bool pad = k >= DP;
             if (HPASS) {
-                if (!T16 && pad) s[j * TF + k] = INF;
+                if (!T16 && (pad || (MODE == SPREAD && k >= D))) s[j * TF + k] = INF;
                 if (pad || !use_phi) s[OP + j * VF + k] = 0.0f;
             } else if (pad) {
                 s[OP + j * VF + k] = INF;
@@ -512,7 +557,6 @@ __global__ void __launch_bounds__(PAIRED ? 64 : 128) k_crf_chain(const CrfPassAr
     }
     __syncwarp();
 
-    const int nblk = (n + BLK - 1) / BLK;
     int ibuf = 0; // the buffer of the next copied block
     // copy block b into the next buffer
     auto issue = [&](int b) {
@@ -521,13 +565,17 @@ __global__ void __launch_bounds__(PAIRED ? 64 : 128) k_crf_chain(const CrfPassAr
             const uint32_t d = ring_s + (uint32_t)(ibuf * BF) * 4u;
             const long o = (long)i0 * ns;
             if constexpr (!RAG) {
-                if (HPASS && D == LP) {
-                    if constexpr (T16) copy_run<P, 2>(d, thetaq + o, lane, cnt);
-                    else copy_run<P, 4>(d, theta + o, lane, cnt);
+                if constexpr (HPASS) {
+                    const long to = tcb + (long)i0 * D;
+                    if constexpr (T16) copy_run<P, 2>(d, thetaq + (long)i0 * D, lane, cnt);
+                    else if constexpr (MODE == SPREAD) copy_spread<P>(d, a.theta + to, lane, cnt, D);
+                    else if (D == LP) copy_run<P, 4>(d, a.theta + to, lane, cnt);
+                    else copy_nodes<P>(d, a.theta + to, D, lane, cnt, D);
+                }
+                if (HPASS && DP == LP) {
                     if (use_phi) copy_run<P, 4>(d + OP * 4, phi + o, lane, cnt);
                 } else {
-                    if (HPASS) copy_nodes<P>(d, theta + o, ns, lane, cnt, D);
-                    if (use_phi) copy_nodes<P>(d + OP * 4, phi + o, ns, lane, cnt, D);
+                    if (use_phi) copy_nodes<P>(d + OP * 4, phi + o, ns, lane, cnt, DP);
                 }
             } else {
                 const long total = (long)W * H * D * a.np;
@@ -618,7 +666,7 @@ __global__ void __launch_bounds__(PAIRED ? 64 : 128) k_crf_chain(const CrfPassAr
         const float *ec = ms + BLK * LP;
 #pragma unroll
         for (int r = 0; r < P; ++r) L[r] = b > 0 ? Lc[r] : 0.0f;
-        if (b > 1) load_vec<P, VEC>(lbuf + (long)(b - 1) * BLK * ns, lane, D, Lc);
+        if (b > 1) load_vec<P, VEC>(lbuf + (b - 1) * ls, lane, DP, Lc);
         read_node(bs, i0, 0, nxt);
         read_edge(ec, 1, nxt);
         auto again = [&](int j, bool more) { // more: another node follows in the block
@@ -658,7 +706,7 @@ __global__ void __launch_bounds__(PAIRED ? 64 : 128) k_crf_chain(const CrfPassAr
         cp_wait<0>();
         meet(); // the first messages are in memory
         for (int q = 0; q < NB - 1; ++q) issue(nblk - 1 - q);
-        if (nblk > 1) load_vec<P, VEC>(lbuf + (long)(nblk - 1) * BLK * ns, lane, D, Lc);
+        if (nblk > 1) load_vec<P, VEC>(lbuf + (nblk - 1) * ls, lane, DP, Lc);
         wn = weights(nblk - 1), ms = msg;
         for (int b = nblk - 1; b >= 0; --b) {
             edge_costs(wn, ms + BLK * LP);
@@ -683,7 +731,7 @@ __global__ void __launch_bounds__(PAIRED ? 64 : 128) k_crf_chain(const CrfPassAr
     if (!PAIRED)
         for (int b = 0; b < NB - 1; ++b) issue(b);
     float wn = PAIRED ? 0.0f : weights(0), *ms = msg;
-    long so = 0; // element offset of the node being stored
+    long so = 0; // element offset of the message being stored, then of the node's phi
     for (int b = 0; b < nblk; ++b) {
         meet();
         if (!PAIRED) {
@@ -699,8 +747,8 @@ __global__ void __launch_bounds__(PAIRED ? 64 : 128) k_crf_chain(const CrfPassAr
             __syncwarp();
         }
         const int i0 = b * BLK, cnt = min(BLK, n - i0), gl = lane - (i0 & 31);
-        if (b > 0) write_vec<P, VEC>(lbuf + so, lane, D, L);
-        so += BLK * ns;
+        if (b > 0) write_vec<P, VEC>(lbuf + so, lane, DP, L);
+        so += ls;
         read_node(bs, i0, 0, nxt);
         read_edge(ec, 1, nxt);
         auto step = [&](int j, bool more, bool last) { // more: node j + 1 is in the block
@@ -738,10 +786,10 @@ __global__ void __launch_bounds__(PAIRED ? 64 : 128) k_crf_chain(const CrfPassAr
     };
     __syncwarp();
     meet();
-    const int Dst = a.store_phi ? D : 0; // labels of phi to store
+    const int Dst = a.store_phi ? DP : 0; // labels of phi to store
     if (!PAIRED) {
         for (int q = 0; q < NB - 1; ++q) issue(nblk - 1 - q);
-        if (nblk > 1) load_vec<P, VEC>(lbuf + (long)(nblk - 1) * BLK * ns, lane, D, Lc);
+        if (nblk > 1) load_vec<P, VEC>(lbuf + (nblk - 1) * ls, lane, DP, Lc);
         wn = weights(nblk - 1);
     }
     ms = msg;
@@ -809,13 +857,13 @@ __global__ void __launch_bounds__(PAIRED ? 64 : 128) k_crf_chain(const CrfPassAr
     if (lane == 0) a.cmin[(long)nch * pair + chain] = cmin;
 }
 
-template <int P, int DELTA, bool HPASS, bool T16, bool RAGGED, bool PAIRED>
+template <int P, int DELTA, bool HPASS, bool T16, int MODE, bool PAIRED>
 int launch_form_as(const CrfPassArgs &a, const CrfForm &f, cudaStream_t st)
 {
     const int wpb = PAIRED ? 1 : f.wpb;
-    const size_t sm = sizeof(float) * wpb * (size_t)chain_floats(P, HPASS, T16, RAGGED, PAIRED, f.buffers);
+    const size_t sm = sizeof(float) * wpb * (size_t)chain_floats(P, HPASS, T16, MODE, PAIRED, f.buffers);
     if (sm > 227 * 1024) return fail(CNNCRF_EUNSUPPORTED, "crf: %zu bytes of ring per CTA", sm);
-    auto kern = k_crf_chain<P, DELTA, HPASS, T16, RAGGED, PAIRED>;
+    auto kern = k_crf_chain<P, DELTA, HPASS, T16, MODE, PAIRED>;
     CNNCRF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     const long chains = (long)(HPASS ? a.H : a.W) * a.np;
     {
@@ -826,18 +874,26 @@ int launch_form_as(const CrfPassArgs &a, const CrfForm &f, cudaStream_t st)
     return CNNCRF_OK;
 }
 
+template <int P, int DELTA, bool HPASS, bool T16, int MODE>
+int launch_mode(const CrfPassArgs &a, const CrfForm &f, cudaStream_t st)
+{
+    return f.paired ? launch_form_as<P, DELTA, HPASS, T16, MODE, true>(a, f, st)
+                    : launch_form_as<P, DELTA, HPASS, T16, MODE, false>(a, f, st);
+}
+
 template <int P, int DELTA, bool HPASS, bool T16>
 int launch_form(const CrfPassArgs &a, const CrfForm &f, cudaStream_t st)
 {
     // whole 16-byte chunks where the vectors allow them (the solver's arrays start on 16 bytes: the workspace's by its
     // layout, a caller's cost volume by check_args)
-    if (a.D % 4 == 0)
-        return f.paired ? launch_form_as<P, DELTA, HPASS, T16, false, true>(a, f, st)
-                        : launch_form_as<P, DELTA, HPASS, T16, false, false>(a, f, st);
+    const int mode = vec_mode(a, HPASS);
+    if (mode == ALIGNED) return launch_mode<P, DELTA, HPASS, T16, ALIGNED>(a, f, st);
     if constexpr (T16) return fail(CNNCRF_EINVAL, "crf: 16-bit unary at depth %d", a.D); // crf_reads_q16: never
-    else
-        return f.paired ? launch_form_as<P, DELTA, HPASS, T16, true, true>(a, f, st)
-                        : launch_form_as<P, DELTA, HPASS, T16, true, false>(a, f, st);
+    else {
+        if constexpr (HPASS)
+            if (mode == SPREAD) return launch_mode<P, DELTA, HPASS, T16, SPREAD>(a, f, st);
+        return launch_mode<P, DELTA, HPASS, T16, RAGGED>(a, f, st);
+    }
 }
 
 template <int P, int DELTA> int launch_dir(const CrfPassArgs &a, bool hpass, const CrfForm &f, cudaStream_t st)

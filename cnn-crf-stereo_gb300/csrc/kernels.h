@@ -213,7 +213,7 @@ int edge_weights(const float *gray, int W, int H, float alpha, float beta, float
                  const float *d_gw, float *wx, float *wy, cudaStream_t st);
 int quadfit_direct(float *u, const float *c1, long npx, int D, float dmin, float dstep, cudaStream_t st);
 // the same with C1 = cost (or its 16-bit copy) - phi taken where it is read
-int quadfit_solver(float *u, const float *cost, const void *costq, UnaryQ16 q, const float *phi, long npx, int D, float dmin,
+int quadfit_solver(float *u, const float *cost, const void *costq, UnaryQ16 q, const float *phi, int DP, long npx, int D, float dmin,
                    float dstep, cudaStream_t st);
 int lr_check(const float *left, const float *right, int W, int H, float th, float *out, cudaStream_t st);
 
@@ -252,11 +252,11 @@ bool crf_reads_q16(int D);
 // the slack_prop_2D_alg object of the C ABI reads costq instead of its cost when set
 void slackprop_set_costq(struct ::cnncrf_slackprop *sp, const void *costq, UnaryQ16 q);
 // quadfit_direct on the last solve's C1 without writing it out; the object's form fails as get_C1 does before a solve
-int crf_quadfit(float *u, const float *cost, const void *ws, long npx, int D, float dmin, float dstep, cudaStream_t st,
+int crf_quadfit(float *u, const float *cost, const void *ws, int W, int H, int D, float dmin, float dstep, cudaStream_t st,
                 const void *costq, UnaryQ16 q);
 int slackprop_quadfit(struct ::cnncrf_slackprop *sp, float *u, float dmin, float dstep);
 // theta - phi of the last solve (get_C1); costq: the 16-bit copy that solve read, if any
-int crf_c1(const float *cost, const void *ws, long n, float *out, cudaStream_t st, int D = 0,
+int crf_c1(const float *cost, const void *ws, int W, int H, int D, float *out, cudaStream_t st,
            const void *costq = nullptr, UnaryQ16 q = UnaryQ16{0.0f, 0.0f});
 
 // CRF tile: prefetch depth (4: two blocks of nodes, 8: three where shared memory

@@ -51,7 +51,7 @@ int cnncrf::k::slackprop_quadfit(cnncrf_slackprop *sp, float *u, float dmin, flo
 {
     if (!sp || !u) return fail(CNNCRF_EINVAL, "null argument");
     if (!sp->ran || sp->ops.total_it <= 0) return fail(CNNCRF_ESTATE, "slackprop: get_C1 before execute");
-    return k::crf_quadfit(u, sp->cost, sp->ws.get(), (long)sp->W * sp->H, sp->D, dmin, dstep, sp->st, sp->costq, sp->q);
+    return k::crf_quadfit(u, sp->cost, sp->ws.get(), sp->W, sp->H, sp->D, dmin, dstep, sp->st, sp->costq, sp->q);
 }
 
 extern "C" {
@@ -257,7 +257,7 @@ int cnncrf_slackprop_get_c1(cnncrf_slackprop_t sp, float **d_c1)
     if (!sp->ran || sp->ops.total_it <= 0) return fail(CNNCRF_ESTATE, "slackprop: get_C1 before execute");
     long n = (long)sp->W * sp->H * sp->D;
     CNNCRF_TRY(sp->c1.reserve(sizeof(float) * n));
-    CNNCRF_TRY(k::crf_c1(sp->cost, sp->ws.get(), n, sp->c1.as<float>(), sp->st, sp->D, sp->costq, sp->q));
+    CNNCRF_TRY(k::crf_c1(sp->cost, sp->ws.get(), sp->W, sp->H, sp->D, sp->c1.as<float>(), sp->st, sp->costq, sp->q));
     *d_c1 = sp->c1.as<float>();
     return CNNCRF_OK;
 }

@@ -48,3 +48,26 @@ def test_chain_counts(cuda, oracle, H, W, D):
 def test_redundant_offsets(cuda, oracle, L1, L2, delta, shape, D):
     """rho at the far offsets reaches L2 (or just does not): the kernels leave them out (or not)."""
     check(cuda, oracle, 17, 21, D, L1, L2, delta, shape, iters=3)
+
+
+# the solver's phi at a pitch of whole chunks (or not: few labels, images a few pixels wide), read back as C1
+@pytest.mark.parametrize("D", [1, 2, 3, 5, 30, 63, 75, 97, 190, 255])
+@pytest.mark.parametrize("H,W", [(1, 9), (9, 2), (17, 40), (3, 1300)])
+def test_c1_of_any_pitch(cuda, oracle, H, W, D):
+    torch = cuda
+    from cnncrf.api import SlackProp
+    rng = np.random.default_rng(H * 1000 + D)
+    cost = rng.random((H, W, D)).astype(np.float32)
+    wx, wy = ((rng.random((H, W)) * 0.5).astype(np.float32) for _ in range(2))
+    olab, olb, _, oc1 = oracle.crf(cost, wx, wy, 0.5, 1.5, 3, 3, shape=1, want_c1=True)
+    d = [torch.from_numpy(x).cuda() for x in (cost, wx, wy)]
+    labels = torch.zeros((H, W), device="cuda", dtype=torch.int32)
+    sp = SlackProp()
+    sp.init(d[0], labels)
+    for k, v in (("L1", 0.5), ("L2", 1.5), ("delta", 3), ("total_it", 3), ("shape", 1)):
+        sp.ops[k] = v
+    sp.update_W(d[1], d[2])
+    for _ in range(2):  # the second solve starts on what the first left behind
+        sp.execute()
+        assert np.array_equal(labels.cpu().numpy(), olab) and sp.LB() == olb
+        assert np.array_equal(sp.get_C1().cpu().numpy(), oc1)
