@@ -200,46 +200,60 @@ template <int P, int DELTA> struct Edge {
     }
 };
 
-// out = minconv(v) - g with out_k = min(v_k, v_{k+-t} + w rho_t (t <= DELTA), g + w L2) - g, g = min v; cw: the edge's
-// w L2, w rho_1, ..
+// out = minconv(v) - g with out_k = min(v_k, v_{k+-t} + w rho_t (t <= DELTA), g + w L2) - g; returns g = min v.  cw: the
+// edge's w L2, w rho_1, ..  This is the chain's critical path: the neighbours' labels are sent off first, the minimum and
+// what a lane's own labels give are worked out while they travel, and an arriving label takes one addition, of its cost
+// with the edge constant in it, and one minimum.
 template <int P, int DELTA>
-__device__ __forceinline__ void minconv(const float (&v)[P], float g, const float (&cw)[EDGE], const Edge<P, DELTA> &ed,
-                                        float (&out)[P])
+__device__ __forceinline__ float minconv(const float (&v)[P], const float (&cw)[EDGE], const Edge<P, DELTA> &ed, float (&out)[P])
 {
-    constexpr int HL = (DELTA + 1) / 2 * 2; // halo, whole pairs: E[HL + i] = value at label lane P + i
-    constexpr int NE = P + 2 * HL + (P & 1);
-    float E[NE];
-#pragma unroll
-    for (int i = 0; i < P; ++i) E[HL + i] = v[i];
+    float lo[DELTA + 1], hi[DELTA + 1]; // labels lane P - t and lane P + P - 1 + t
 #pragma unroll
     for (int t = 1; t <= DELTA; ++t) {
-        const int ol = (t + P - 1) / P, rl = (P - t % P) % P;          // label lane P - t
-        const int oh = (P - 1 + t) / P, rh = (P - 1 + t) % P;          // label lane P + P - 1 + t
-        E[HL - t] = __fadd_rn(__shfl_up_sync(0xffffffffu, v[rl], ol), ed.lo[ol]);
-        E[HL + P - 1 + t] = __fadd_rn(__shfl_down_sync(0xffffffffu, v[rh], oh), ed.hi[oh]);
+        const int ol = (t + P - 1) / P, rl = (P - t % P) % P;
+        const int oh = (P - 1 + t) / P, rh = (P - 1 + t) % P;
+        lo[t] = __shfl_up_sync(0xffffffffu, v[rl], ol);
+        hi[t] = __shfl_down_sync(0xffffffffu, v[rh], oh);
     }
-    float o[P];
+    const float g = warp_min<P>(v), base = __fadd_rn(g, cw[0]);
+    float o[P], pend[P]; // pend: a value not yet in the minimum o, so that they go in by pairs
+    bool has[P];
 #pragma unroll
-    for (int r = 0; r < P; ++r) o[r] = v[r];
+    for (int r = 0; r < P; ++r) o[r] = v[r], pend[r] = INF, has[r] = false;
+    auto put = [&](int r, float x) {
+        if (has[r]) o[r] = min3(o[r], pend[r], x);
+        else pend[r] = x;
+        has[r] = !has[r];
+    };
 #pragma unroll
     for (int t = 1; t <= DELTA; ++t) {
-        const float c = cw[t];
-        // S[j] = E[j] + c where some label reads it: labels -t .. P-1-t and t .. P-1+t
-        float S[NE];
-        auto need = [](int i, int tt) { return (i >= -tt && i <= P - 1 - tt) || (i >= tt && i <= P - 1 + tt); };
+        float S[P + 1];
 #pragma unroll
-        for (int i = -HL; i < P + HL; i += 2) {
-            if (need(i, t) && need(i + 1, t)) add2(E[HL + i], E[HL + i + 1], c, c, S[HL + i], S[HL + i + 1]);
-            else if (need(i, t)) S[HL + i] = __fadd_rn(E[HL + i], c);
-            else if (need(i + 1, t)) S[HL + i + 1] = __fadd_rn(E[HL + i + 1], c);
+        for (int i = 0; i < P; i += 2) {
+            if (i + 1 < P) add2(v[i], v[i + 1], cw[t], cw[t], S[i], S[i + 1]);
+            else S[i] = __fadd_rn(v[i], cw[t]);
         }
 #pragma unroll
-        for (int r = 0; r < P; ++r) o[r] = min3(o[r], S[HL + r - t], S[HL + r + t]);
+        for (int r = 0; r < P; ++r) {
+            if (r - t >= 0) put(r, S[r - t]);
+            if (r + t < P) put(r, S[r + t]);
+        }
     }
-    const float base = __fadd_rn(g, cw[0]);
 #pragma unroll
-    for (int r = 0; r < P; ++r) o[r] = fminf(o[r], base);
+    for (int r = 0; r < P; ++r) put(r, base);
+#pragma unroll
+    for (int t = 1; t <= DELTA; ++t)
+#pragma unroll
+        for (int q = 1; q <= t; ++q) { // the label q beyond the lane's, t from label r
+            const int ol = (q + P - 1) / P, oh = (P - 1 + q) / P;
+            if (t - q < P) put(t - q, __fadd_rn(lo[q], __fadd_rn(cw[t], ed.lo[ol])));
+            if (t - q < P) put(P - 1 - (t - q), __fadd_rn(hi[q], __fadd_rn(cw[t], ed.hi[oh])));
+        }
+#pragma unroll
+    for (int r = 0; r < P; ++r)
+        if (has[r]) o[r] = fminf(o[r], pend[r]);
     vsub1<P>(o, g, out);
+    return g;
 }
 
 // ---------------------------------------------------------------- copies
@@ -496,12 +510,15 @@ template <int P, bool ALIGNED> __device__ __forceinline__ void load_vec(const fl
 // What bounds it: many chains, DRAM (eight KITTI pairs at D = 128: the H pass
 // 7.9 GB in 1.18 ms, 6.7 TB/s, and the V pass 6.2 GB in 0.93 ms; with all
 // messages stored and read back 1.72 and 1.38 ms).  Few chains, the latency of
-// a node's step, about 430 cycles for both sweeps of a KITTI pair's row: four
+// a node's step, about 420 cycles for both sweeps of a KITTI pair's row: four
 // halo shuffles issue 4.3 cycles apart and return after 24, the warp minimum
 // after 18, and the copies of a block cost 18 cycles per instruction, which is
-// why they are few and on the second warp (one pair's H pass 470 -> 258 us,
-// its V pass 208 -> 161 us; the 256 x 192, D = 32 solve's 89 -> 40 and 70 ->
-// 34 us).  Measured and left out: bulk copies on mbarriers for the H blocks
+// why they are few and on the second warp (one pair's H pass 470 -> 252 us,
+// its V pass 208 -> 154 us; the 256 x 192, D = 32 solve's 89 -> 39 and 70 ->
+// 32 us).  The first warp's sweeps bound it: the forward one takes 160 to 185
+// cycles a node, the backward one 200 to 230, as long without the second
+// warp's recomputation.  Sending the halo off before the warp minimum gave 2
+// to 5 % (256 x 192, D = 128: 48.6 -> 46.2 and 39.9 -> 38.5 us).  Measured and left out: bulk copies on mbarriers for the H blocks
 // (a wait costs 150 cycles, cp.async's 43; 338 against 316 us for one pair),
 // and keeping all messages for few chains (276 against 258 us).
 template <int P, int DELTA, bool HPASS, bool T16, int MODE, bool PAIRED>
@@ -678,8 +695,7 @@ __global__ void __launch_bounds__(PAIRED ? 64 : 128) k_crf_chain(const CrfPassAr
             vadd<P>(L, cur.un, v);
             write_vec<P, true>(ms + j * LP, lane, LP, v);
             if (more) {
-                const float g = warp_min<P>(v);
-                minconv<P, DELTA>(v, g, cur.cw, ed, L);
+                minconv<P, DELTA>(v, cur.cw, ed, L);
             }
         };
         if (cnt == BLK) {
@@ -758,9 +774,8 @@ __global__ void __launch_bounds__(PAIRED ? 64 : 128) k_crf_chain(const CrfPassAr
                 read_edge(ec, j + 2, nxt);
             }
             vadd<P>(L, cur.un, v);
-            const float g = warp_min<P>(v);
+            const float g = last ? warp_min<P>(v) : minconv<P, DELTA>(v, cur.cw, ed, L);
             gb = gl == j ? g : gb;
-            if (!last) minconv<P, DELTA>(v, g, cur.cw, ed, L);
         };
         if (b < nblk - 1) {
 #pragma unroll
@@ -837,8 +852,7 @@ __global__ void __launch_bounds__(PAIRED ? 64 : 128) k_crf_chain(const CrfPassAr
             so -= ns;
             if (!first) {
                 vadd<P>(A, R, v);
-                const float g = warp_min<P>(v);
-                minconv<P, DELTA>(v, g, cur.cw, ed, R);
+                minconv<P, DELTA>(v, cur.cw, ed, R);
             }
         };
         so = (long)(i0 + cnt - 1) * ns;
