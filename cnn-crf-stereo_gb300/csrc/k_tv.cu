@@ -50,13 +50,15 @@ constexpr int KMAX = 5;
 __device__ __forceinline__ float clampf(float v, float lo, float hi) { return fmaxf(lo, fminf(v, hi)); }
 
 // prox_p with alpha = 0 (stereo/stereo.cu:752-757): v itself where |v| <= 0 w, else the shrunk |v| with v's sign,
-// clamped.  With beta >= 0 the first case needs no test of its own: a zero shrinks to a zero of its sign
+// clamped.  With beta >= 0 the first case is v = 0 alone: any other |v| <= 0 w shrinks to a zero that the clamp leaves.  The
+// zero itself must not reach the clamp, which a negative w turns into |w| (4096 x 2160, ten iterations: 522 us with the
+// test, 516 without; a vote per tile for weights without negative ones 523)
 template <bool BETA_POS> __device__ __forceinline__ float prox_p0(float v, float beta, float sigma, float w)
 {
     if (!BETA_POS && fabsf(v) <= __fmul_rn(w, 0.0f)) return v;
     const float m = fmaxf(0.0f, __fmaf_rn(-sigma, beta, fabsf(v)));
     const float r = BETA_POS ? copysignf(m, v) : __fmul_rn(m, v > 0.0f ? 1.0f : -1.0f);
-    return clampf(r, -w, w);
+    return BETA_POS && v == 0.0f ? v : clampf(r, -w, w);
 }
 
 struct TvArgs {
