@@ -30,7 +30,7 @@
 //
 // Bound by instruction issue: three IEEE divisions, two prox operators and
 // the clamps per pixel and iteration, on 1.7 times the interior's pixels at K
-// = 5.  Ten iterations on 4096 x 2160: 787 -> 516 us (a thread had four pixels
+// = 5.  Ten iterations on 4096 x 2160: 787 -> 521 us (a thread had four pixels
 // eight rows apart, every neighbour through shared memory with clamped
 // indices).  Larger tiles lose to their barriers what they save in halo: 64 x
 // 64 539 us, 64 x 48 566 us.
@@ -50,15 +50,28 @@ constexpr int KMAX = 5;
 __device__ __forceinline__ float clampf(float v, float lo, float hi) { return fmaxf(lo, fminf(v, hi)); }
 
 // prox_p with alpha = 0 (stereo/stereo.cu:752-757): v itself where |v| <= 0 w, else the shrunk |v| with v's sign,
-// clamped.  With beta >= 0 the first case is v = 0 alone: any other |v| <= 0 w shrinks to a zero that the clamp leaves.  The
-// zero itself must not reach the clamp, which a negative w turns into |w| (4096 x 2160, ten iterations: 522 us with the
-// test, 516 without; a vote per tile for weights without negative ones 523)
+// clamped.  The first case is v = 0 alone (w infinite or NaN apart); with beta >= 0 a zero also shrinks to a zero, but it
+// must not reach the clamp, which a negative w turns into |w| (4096 x 2160, ten iterations: 521 us with the test, 515
+// without; a vote per tile on whether any weight is negative 523)
 template <bool BETA_POS> __device__ __forceinline__ float prox_p0(float v, float beta, float sigma, float w)
 {
     if (!BETA_POS && fabsf(v) <= __fmul_rn(w, 0.0f)) return v;
     const float m = fmaxf(0.0f, __fmaf_rn(-sigma, beta, fabsf(v)));
     const float r = BETA_POS ? copysignf(m, v) : __fmul_rn(m, v > 0.0f ? 1.0f : -1.0f);
     return BETA_POS && v == 0.0f ? v : clampf(r, -w, w);
+}
+
+// a + a - b for two values, each operation rounded by itself: a fused 2 a - b would not overflow where 2 a does
+__device__ __forceinline__ void twice_less(const float (&a)[2], const float (&b)[2], float (&d)[2])
+{
+    asm("{\n\t.reg .b64 ra, rb, rd;\n\t"
+        "mov.b64 ra, {%2, %3};\n\t"
+        "mov.b64 rb, {%4, %5};\n\t"
+        "add.rn.f32x2 rd, ra, ra;\n\t"
+        "sub.rn.f32x2 rd, rd, rb;\n\t"
+        "mov.b64 {%0, %1}, rd;\n\t}"
+        : "=f"(d[0]), "=f"(d[1])
+        : "f"(a[0]), "f"(a[1]), "f"(b[0]), "f"(b[1]));
 }
 
 struct TvArgs {
@@ -131,6 +144,7 @@ __device__ __forceinline__ void tv_tile(const TvArgs &a, int ex, int ey, float2 
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const float left = __shfl_up_sync(0xffffffffu, X[i][1], 1);
+            float u2[2];
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
                 float xl = j ? X[i][0] : left, yu = i ? Y[0][j] : (j ? above.y : above.x);
@@ -142,9 +156,10 @@ __device__ __forceinline__ void tv_tile(const TvArgs &a, int ex, int ey, float2 
                 float un = __fmaf_rn(a.tau, div, u[i][j]);
                 const float num = __fmaf_rn(-a.tau, inn[i][j], un);
                 un = clampf(__fdiv_rn(num, den[i][j]), lo[i][j], hi[i][j]);
-                ub[i][j] = __fmaf_rn(2.0f, un, -u[i][j]); // 2 un is exact
-                u[i][j] = un;
+                u2[j] = un;
             }
+            twice_less(u2, u[i], ub[i]);
+            u[i][0] = u2[0], u[i][1] = u2[1];
         }
         sU[wr][lane] = make_float2(ub[0][0], ub[0][1]); // the warp above reads this warp's upper row
         __syncthreads();
