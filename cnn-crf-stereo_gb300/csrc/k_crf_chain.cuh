@@ -168,23 +168,29 @@ template <int P> __device__ __forceinline__ void vmul1(const float (&a)[P], floa
 // The warp minimum of the lanes' minima: one redux.sync.min.f32 (sm_100 and
 // later), exact like a float min.  A zero may come back with either sign,
 // which no later operation distinguishes (the labels compare values, the
-// bound adds them).  The +inf operand turns a lane of pad labels, which the
-// slack hand-over leaves at NaN, into +inf.
-template <int P> __device__ __forceinline__ float warp_min(const float (&v)[P])
+// bound adds them).  `none`: what pad labels stand for, +inf or NaN
+// (pad_value); it turns a lane of pads, which the slack hand-over leaves at
+// NaN, back into +inf.
+template <int P> __device__ __forceinline__ float warp_min(const float (&v)[P], float none)
 {
     float m;
-    if constexpr (P == 1) m = fminf(v[0], INF);
-    else if constexpr (P == 2) m = min3(v[0], v[1], INF);
+    if constexpr (P == 1) m = fminf(v[0], none);
+    else if constexpr (P == 2) m = min3(v[0], v[1], none);
     else {
         m = min3(v[0], v[1], v[2]);
 #pragma unroll
         for (int r = 3; r + 1 < P; r += 2) m = min3(m, v[r], v[r + 1]);
-        if constexpr (P % 2 == 0) m = min3(m, v[P - 1], INF);
+        if constexpr (P % 2 == 0) m = min3(m, v[P - 1], none);
     }
     float w;
     asm("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(w) : "f"(m));
     return w;
 }
+
+// The value of pad labels.  A minimum takes its other operand either way; where no label has a finite cost, +inf makes the
+// minimum +inf, and NaN leaves it NaN as it is without pads.  So the label counts that fill their lanes at 1, 2, 3, 4, 6 or
+// 8 labels each have NaN (96 labels run in lanes of 4)
+__device__ __forceinline__ float pad_value(int D) { return D % 32 == 0 && D != 160 && D != 224 ? CUDART_NAN_F : INF; }
 
 // Lane constants: 0, or +inf in the lanes whose neighbour `o` lanes below
 // (lo) or above (hi) is outside the warp.  Added to a neighbour's value they
@@ -193,7 +199,8 @@ template <int P> __device__ __forceinline__ float warp_min(const float (&v)[P])
 template <int P, int DELTA> struct Edge {
     static constexpr int NO = (DELTA + P - 1) / P;
     float lo[NO + 1], hi[NO + 1];
-    __device__ __forceinline__ explicit Edge(int lane)
+    float none; // warp_min's
+    __device__ __forceinline__ Edge(int lane, float pad) : none(pad)
     {
 #pragma unroll
         for (int o = 1; o <= NO; ++o) lo[o] = lane < o ? INF : 0.0f, hi[o] = lane + o > 31 ? INF : 0.0f;
@@ -215,7 +222,7 @@ __device__ __forceinline__ float minconv(const float (&v)[P], const float (&cw)[
         lo[t] = __shfl_up_sync(0xffffffffu, v[rl], ol);
         hi[t] = __shfl_down_sync(0xffffffffu, v[rh], oh);
     }
-    const float g = warp_min<P>(v), base = __fadd_rn(g, cw[0]);
+    const float g = warp_min<P>(v, ed.none), base = __fadd_rn(g, cw[0]);
     float o[P], pend[P]; // pend: a value not yet in the minimum o, so that they go in by pairs
     bool has[P];
 #pragma unroll
@@ -556,19 +563,20 @@ __global__ void __launch_bounds__(PAIRED ? 64 : 128) k_crf_chain(const CrfPassAr
     const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring);
     const bool use_phi = !(HPASS && a.first);
 
-    // Labels DP..32 P - 1 (of a SPREAD unary D..) are pads at +inf: set once,
+    // Labels DP..32 P - 1 (of a SPREAD unary D..) are pads: set once,
     // the copies never write them (RAGGED slots hold other vectors' labels
     // there, and read_node masks them).  The first H pass copies no phi: zero.
+    const float none = pad_value(D);
     if (helps && (D < LP || !use_phi)) {
         for (int i = lane; i < NB * BLK * VF; i += 32) {
             const int nd = i / VF, k = i - nd * VF, q = nd / BLK, j = nd - q * BLK;
             float *s = ring + q * BF;
             const bool pad = k >= DP;
             if (HPASS) {
-                if (!T16 && (pad || (MODE == SPREAD && k >= D))) s[j * TF + k] = INF;
+                if (!T16 && (pad || (MODE == SPREAD && k >= D))) s[j * TF + k] = none;
                 if (pad || !use_phi) s[OP + j * VF + k] = 0.0f;
             } else if (pad) {
-                s[OP + j * VF + k] = INF;
+                s[OP + j * VF + k] = none;
             }
         }
     }
@@ -665,7 +673,7 @@ __global__ void __launch_bounds__(PAIRED ? 64 : 128) k_crf_chain(const CrfPassAr
         if (DELTA > 3) nd.cw[4] = ec[j * EDGE + 4];
     };
 
-    const Edge<P, DELTA> ed(lane);
+    const Edge<P, DELTA> ed(lane, none);
     float L[P], v[P];
     Node cur, nxt;
 #pragma unroll
@@ -774,7 +782,7 @@ __global__ void __launch_bounds__(PAIRED ? 64 : 128) k_crf_chain(const CrfPassAr
                 read_edge(ec, j + 2, nxt);
             }
             vadd<P>(L, cur.un, v);
-            const float g = last ? warp_min<P>(v) : minconv<P, DELTA>(v, cur.cw, ed, L);
+            const float g = last ? warp_min<P>(v, none) : minconv<P, DELTA>(v, cur.cw, ed, L);
             gb = gl == j ? g : gb;
         };
         if (b < nblk - 1) {
@@ -834,7 +842,7 @@ __global__ void __launch_bounds__(PAIRED ? 64 : 128) k_crf_chain(const CrfPassAr
             cur = nxt;
             if (j > 0) read_back(j - 1);
             vadd<P>(cur.vm, R, m);
-            const float mu = warp_min<P>(m);
+            const float mu = warp_min<P>(m, none);
             if (!HPASS && want) {
                 int best = 0x7fffffff;
 #pragma unroll
