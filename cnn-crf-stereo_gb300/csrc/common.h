@@ -83,6 +83,16 @@ class DevBuf {
 
 inline int ceil_div(long a, long b) { return (int)((a + b - 1) / b); }
 
+// Shared memory that a CTA can have.
+constexpr size_t SMEM_MAX = 227 * 1024;
+// Lets a kernel's launches take up to SMEM_MAX of dynamic shared memory (it has no static one).  The limit belongs to the
+// kernel and the device, so every thread's launches share it: it is always this value, since a launch's own size would
+// refuse another thread's larger launch between that thread's call and its launch.
+template <class... A> cudaError_t allow_smem(void (*kern)(A...))
+{
+    return cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX);
+}
+
 // Kernel-launch instrumentation.  Every launch site is wrapped in a
 // CNNCRF_PROF scope: it counts the launch, opens an NVTX range named after
 // the kernel in the "cnncrf" domain (a no-op unless a tool such as ncu with

@@ -278,7 +278,7 @@ int census_volume(const float *g1, const float *g2, int W, int H, int fs, const 
     }
     if (whole && W < 1048576 && hi - lo < 8192.0f) {
         const size_t sm = census_bits_smem(fs, D, (int)(hi - lo));
-        if (sm <= 227 * 1024) {
+        if (sm <= SMEM_MAX) {
             const int side = 2 * fs + 1, nw = (side * side - 1 + 31) / 32;
             auto kern = nw == 1   ? k_census_bits<1>
                         : nw == 2 ? k_census_bits<2>
@@ -287,7 +287,7 @@ int census_volume(const float *g1, const float *g2, int W, int H, int fs, const 
                         : nw == 6 ? k_census_bits<6>
                         : nw == 7 ? k_census_bits<7>
                                   : k_census_bits<0>;
-            CNNCRF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+            CNNCRF_CUDA(allow_smem(kern));
             {
                 CNNCRF_PROF("census", st);
                 kern<<<dim3(ceil_div(W, CPX), H), CTH, sm, st>>>(g1, g2, W, H, fs, d_list, D, (int)lo, (int)hi, lambda, vol);

@@ -241,7 +241,7 @@ template <int NP> int launch(FirstParams &p, cudaStream_t st)
     // at most CTAS_PER_SM CTAs per SM (through shared memory): their accumulators fill the SM's 512 TMEM
     // columns, so no CTA waits in its allocation
     const size_t smem = std::max(smem_bytes<NP>(), (size_t)(200 * 1024 / CTAS_PER_SM));
-    CNNCRF_CUDA(cudaFuncSetAttribute(k_conv_first_tc<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CNNCRF_CUDA(allow_smem(k_conv_first_tc<NP>));
     const int grid = std::min(p.num_tiles, CTAS_PER_SM * sms);
     {
         CNNCRF_PROF("conv_first_tc", st);

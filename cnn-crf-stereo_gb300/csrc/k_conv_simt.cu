@@ -658,7 +658,7 @@ __global__ void __launch_bounds__(128, 3) k_conv_patch(ConvArgs a, int npx, int 
 template <int CPW, int TK> int launch_px(const ConvArgs &a, int Ho, int Wo, int K, cudaStream_t st)
 {
     const int sm = 4 * std::max(PXS * px_stage(CPW, TK), 4 * PXT * epi_pitch(CPW));
-    CNNCRF_CUDA(cudaFuncSetAttribute(k_conv_px<CPW, TK>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+    CNNCRF_CUDA(allow_smem(k_conv_px<CPW, TK>));
     CNNCRF_PROF("conv_simt", st);
     k_conv_px<CPW, TK><<<dim3(ceil_div((long)Ho * Wo, PXT), a.n_img), 128, sm, st>>>(a, Ho * Wo, Wo, K);
     return CNNCRF_OK;
@@ -667,7 +667,7 @@ template <int CPW, int TK> int launch_px(const ConvArgs &a, int Ho, int Wo, int 
 template <int CPW, int KP> int launch_patch(const ConvArgs &a, int Ho, int Wo, int K, cudaStream_t st)
 {
     const int sm = 4 * std::max(PXT * KP + K * w_pitch(CPW), 4 * PXT * epi_pitch(CPW));
-    CNNCRF_CUDA(cudaFuncSetAttribute(k_conv_patch<CPW, KP>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+    CNNCRF_CUDA(allow_smem(k_conv_patch<CPW, KP>));
     CNNCRF_PROF("conv_first", st);
     k_conv_patch<CPW, KP><<<dim3(ceil_div((long)Ho * Wo, PXT), a.n_img), 128, sm, st>>>(a, Ho * Wo, Wo, K);
     return CNNCRF_OK;

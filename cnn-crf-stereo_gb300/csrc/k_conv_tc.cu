@@ -727,8 +727,7 @@ template <int NP> int pair_clusters(size_t smem)
     auto it = cache.find(smem);
     if (it != cache.end()) return it->second;
     int n = 0;
-    if (cudaFuncSetAttribute(k_conv_tc<NP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
-        cudaSuccess) {
+    if (allow_smem(k_conv_tc<NP, true>) == cudaSuccess) {
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
@@ -833,7 +832,7 @@ template <int NP> int launch(const TcConvArgs &a, TcParams &p, cudaStream_t st)
         // one cluster per pair of co-resident SMs, each running tile pairs until the list ends
         const int grid = 2 * std::min(nclusters, (p.num_tiles + 1) / 2);
         if (a.bias_splits) *a.bias_splits = 8 * grid;
-        CNNCRF_CUDA(cudaFuncSetAttribute(k_conv_tc<NP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CNNCRF_CUDA(allow_smem(k_conv_tc<NP, true>));
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
@@ -847,7 +846,7 @@ template <int NP> int launch(const TcConvArgs &a, TcParams &p, cudaStream_t st)
     } else {
         const int grid = std::min(p.num_tiles, sms);
         if (a.bias_splits) *a.bias_splits = 8 * grid;
-        CNNCRF_CUDA(cudaFuncSetAttribute(k_conv_tc<NP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CNNCRF_CUDA(allow_smem(k_conv_tc<NP, false>));
         {
             CNNCRF_PROF("conv_tc", st);
             k_conv_tc<NP, false><<<grid, NUM_THREADS, smem, st>>>(ma, ma2, mb, my, mo, p);

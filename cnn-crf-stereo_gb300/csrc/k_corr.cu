@@ -432,7 +432,7 @@ int launch_unit(const float *fl, const float *fr, int H, int W, int C, const flo
     const int KG = (KB + 7) / 8, PX = 8 * PG;
     const int threads = std::max(128, (PG * KG + 31) & ~31); // narrow bands: more warps load than compute
     const size_t sm = unit_smem(PG, C, KB);
-    CNNCRF_CUDA(cudaFuncSetAttribute(k_corr_unit<PG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    CNNCRF_CUDA(allow_smem(k_corr_unit<PG>));
     CNNCRF_PROF("corr", st);
     k_corr_unit<PG><<<dim3(ceil_div(W, PX), H, npairs), threads, sm, st>>>(fl, fr, H, W, C, d_list, D, KG, smax, unary, out,
                                                                            fps);
@@ -454,8 +454,8 @@ static int corr_launch(const TIN *fl, const TIN *fr, int H, int W, int C, int cs
     const size_t tiles = (size_t)C * (PIX + 1) + (size_t)C * (NJ * 32 + 1) + D;
     const size_t tres = (size_t)PIX * (NJ * 32 + 1) + D;
     const size_t band_smem = sizeof(float) * std::max(tiles, tres);
-    if (!interp && NJ <= MAXNJ && band_smem <= 227 * 1024) {
-        CNNCRF_CUDA(cudaFuncSetAttribute(k_corr_band<TIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)band_smem));
+    if (!interp && NJ <= MAXNJ && band_smem <= SMEM_MAX) {
+        CNNCRF_CUDA(allow_smem(k_corr_band<TIN>));
         {
             CNNCRF_PROF("corr", st);
             k_corr_band<TIN><<<grid, 256, band_smem, st>>>(fl, fr, H, W, C, cs, d_list, D, omin, omax, NJ, unary, out,
@@ -466,9 +466,9 @@ static int corr_launch(const TIN *fl, const TIN *fr, int H, int W, int C, int cs
     }
     int R = PIX + omax - omin + 1;
     size_t smem = sizeof(float) * ((size_t)(PIX + R) * (C + 1) + D);
-    if (smem > 227 * 1024)
+    if (smem > SMEM_MAX)
         return fail(CNNCRF_EINVAL, "correlation: disparity band too wide (%zu bytes of shared memory)", smem);
-    CNNCRF_CUDA(cudaFuncSetAttribute(k_corr<TIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CNNCRF_CUDA(allow_smem(k_corr<TIN>));
     {
         CNNCRF_PROF("corr", st);
         k_corr<TIN><<<grid, 256, smem, st>>>(fl, fr, H, W, C, cs, d_list, D, omin, omax, interp ? 1 : 0, unary, out,
@@ -486,12 +486,12 @@ int correlation(const float *fl, const float *fr, int H, int W, int C, const flo
     const int KB = omax - omin + 1;
     const bool al16 = (((uintptr_t)fl | (uintptr_t)fr) & 15) == 0 && C % 4 == 0 && fps % 4 == 0;
     if (!interp && al16 && D <= 256 && KB <= 256 && npairs <= 65535 && H <= 65535) {
-        if (KB <= 64 && unit_smem(16, C, KB) <= 227 * 1024) {
+        if (KB <= 64 && unit_smem(16, C, KB) <= SMEM_MAX) {
             CNNCRF_TRY(launch_unit<16>(fl, fr, H, W, C, d_list, D, KB, omax, unary, out, st, npairs, fps));
             CNNCRF_CHECK_LAUNCH();
             return CNNCRF_OK;
         }
-        if (unit_smem(8, C, KB) <= 227 * 1024) {
+        if (unit_smem(8, C, KB) <= SMEM_MAX) {
             CNNCRF_TRY(launch_unit<8>(fl, fr, H, W, C, d_list, D, KB, omax, unary, out, st, npairs, fps));
             CNNCRF_CHECK_LAUNCH();
             return CNNCRF_OK;

@@ -377,7 +377,7 @@ int launch_side(const void *P, int fs, const float *g, const float *d_list, int 
         if (smem_bytes(s, span, p.grows, p.gstride) <= (size_t)maxsm) p.stages = s;
     if (!p.stages) return fail(CNNCRF_EUNSUPPORTED, "corr_bwd_tc: shared memory");
     const size_t smem = smem_bytes(p.stages, span, p.grows, p.gstride);
-    CNNCRF_CUDA(cudaFuncSetAttribute(k_corr_bwd_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CNNCRF_CUDA(allow_smem(k_corr_bwd_tc));
     k_corr_bwd_tc<<<std::min(p.num_tiles, sms), NUM_THREADS, smem, st>>>(mp, p);
     CNNCRF_CHECK_LAUNCH();
     return CNNCRF_OK;
@@ -390,7 +390,7 @@ bool corr_bwd_tc_supported(int C, int fs, int D, int omin, int omax)
     const int span = omax - omin + 1, gstride = (D + 7) & ~7;
     // two stages beside the right side's gradient window
     return C >= 1 && C <= 128 && fs % 64 == 0 && fs >= ((C + 15) & ~15) && D >= 1 && D <= 32767 &&
-           span <= MAX_SPAN && smem_bytes(2, span, BM - 1 + span, gstride) <= 227 * 1024;
+           span <= MAX_SPAN && smem_bytes(2, span, BM - 1 + span, gstride) <= SMEM_MAX;
 }
 
 int corr_bwd_tc(const void *fl, const void *fr, int fs, const float *gvol, const float *d_list, int npairs, int H,

@@ -476,7 +476,7 @@ int correlation_tc(const void *feat, int npairs, int H, int W, int C, int cp, co
     const size_t smem = smem_bytes(p.stages, D);
     if (smem > (size_t)maxsm) return fail(CNNCRF_EUNSUPPORTED, "correlation_tc: %zu bytes of shared memory", smem);
     auto kern = k_corr_tc<EPI_WARPS>;
-    CNNCRF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CNNCRF_CUDA(allow_smem(kern));
     const int grid = std::min(p.num_tiles, sms);
     {
         CNNCRF_PROF("corr_tc", st);

@@ -183,7 +183,7 @@ int pass(const CrfPassArgs &a, bool hpass, int delta, int ring, int wpb, cudaStr
 // whether a CTA of the smallest form fits (it does for every label count and wpb; an upper bound for the other vector modes)
 bool fits(int D, bool hpass, int wpb)
 {
-    return form_smem(D, hpass, false, RAGGED, CrfForm{false, 2, wpb}) <= 227 * 1024;
+    return form_smem(D, hpass, false, RAGGED, CrfForm{false, 2, wpb}) <= SMEM_MAX;
 }
 
 // the tile of the tuning table for this shape, each pass falling back to the

@@ -884,9 +884,9 @@ int launch_form_as(const CrfPassArgs &a, const CrfForm &f, cudaStream_t st)
 {
     const int wpb = PAIRED ? 1 : f.wpb;
     const size_t sm = sizeof(float) * wpb * (size_t)chain_floats(P, HPASS, T16, MODE, PAIRED, f.buffers);
-    if (sm > 227 * 1024) return fail(CNNCRF_EUNSUPPORTED, "crf: %zu bytes of ring per CTA", sm);
+    if (sm > SMEM_MAX) return fail(CNNCRF_EUNSUPPORTED, "crf: %zu bytes of ring per CTA", sm);
     auto kern = k_crf_chain<P, DELTA, HPASS, T16, MODE, PAIRED>;
-    CNNCRF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    CNNCRF_CUDA(allow_smem(kern));
     const long chains = (long)(HPASS ? a.H : a.W) * a.np;
     {
         CNNCRF_PROF(HPASS ? "crf_h" : "crf_v", st);

@@ -938,7 +938,7 @@ static int corr_bwd_t(const T *fl, const T *fr, int fs, const float *gvol, const
         const int band = omax - omin + 1, Cs = (C + 3) & ~3;
         const size_t sm = corr_bwd_blk_smem(band, Cs, sizeof(T), D);
         if (sm <= (size_t)maxsm) {
-            CNNCRF_CUDA(cudaFuncSetAttribute(k_corr_bwd_blk<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+            CNNCRF_CUDA(allow_smem(k_corr_bwd_blk<T>));
             const dim3 g(ceil_div(W, CB_TX), H, npairs);
             {
                 CNNCRF_PROF("corr_bwd", st);
@@ -951,9 +951,9 @@ static int corr_bwd_t(const T *fl, const T *fr, int fs, const float *gvol, const
     }
     const int span = 32 + omax - omin;
     const size_t smem = sizeof(float) * (size_t)span * C + sizeof(int) * (size_t)D;
-    if (smem > 227 * 1024) return fail(CNNCRF_EUNSUPPORTED, "corr_bwd: band %d too wide", omax - omin);
-    CNNCRF_CUDA(cudaFuncSetAttribute(k_corr_bwd_left<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CNNCRF_CUDA(cudaFuncSetAttribute(k_corr_bwd_right<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > SMEM_MAX) return fail(CNNCRF_EUNSUPPORTED, "corr_bwd: band %d too wide", omax - omin);
+    CNNCRF_CUDA(allow_smem(k_corr_bwd_left<T>));
+    CNNCRF_CUDA(allow_smem(k_corr_bwd_right<T>));
     const dim3 g(ceil_div(W, 32), H, npairs);
     {
         CNNCRF_PROF("corr_bwd", st);

@@ -331,7 +331,7 @@ int wgrad_tc(const void *dzpad, int Cout, int cpa, const void *in, long in_pix, 
         if (smem_bytes(s) <= (size_t)maxsm) p.stages = s;
     if (!p.stages) return fail(CNNCRF_EUNSUPPORTED, "wgrad_tc: shared memory");
     const size_t smem = smem_bytes(p.stages);
-    CNNCRF_CUDA(cudaFuncSetAttribute(k_wgrad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CNNCRF_CUDA(allow_smem(k_wgrad_tc));
     // every split has at least one step: splits <= steps and steps_per_split = ceil(steps / splits)
     const int used = (int)((steps + p.steps_per_split - 1) / p.steps_per_split);
     {
