@@ -162,6 +162,19 @@ size_t census_bits_smem(int fs, int D, int range)
     return 4 * (side * (CPX + cols + 4 * fs) + nw * (CPX + cols) + bits + 1 + D);
 }
 
+// Whether the bit strings are the cheaper way.  A CTA's 64 pixels take 2 CPX + range strings of side^2 comparisons however
+// few the labels are, k_census D times side^2 comparisons per pixel (720 x 480 at filter size 7: 112 us plus 0.5 us per
+// column of range against 16 us plus 96 us per label; three labels 1000 columns apart 2514 against 303 us, four labels in a
+// row at filter size 1 40 against 28 us).  The line, from filter sizes 1 to 16, 1 to 16 labels and ranges up to 8000, lies
+// where no list is slower than in k_census; strings cost 1.3 and 2 times as much with two and one CTAs per SM
+bool bits_pay(int fs, int D, int range, size_t smem)
+{
+    const double sq = (2 * fs + 1) * (2 * fs + 1);
+    const size_t ctas = 228 * 1024 / (smem + 1024);
+    const double strings = (2 * CPX + range) * (ctas >= 3 ? 1.0 : (ctas == 2 ? 1.3 : 2.0));
+    return strings * (sq + 2) + 8000 < 140 * sq * D;
+}
+
 // separable Gaussian, radius R, clamp-to-edge; horizontal then vertical pass
 __global__ void k_gauss_h(const float *__restrict__ in, int W, int H, const float *__restrict__ w, int R,
                           float *__restrict__ out)
@@ -269,7 +282,7 @@ int census_volume(const float *g1, const float *g2, int W, int H, int fs, const 
                   float lambda, float *vol, cudaStream_t st)
 {
     if (fs < 1 || fs > 16) return fail(CNNCRF_EINVAL, "census: filter size %d outside 1..16", fs);
-    // k_census_bits: integer disparities whose coordinates x + dx + 0.5 - d are exact, and tiles that fit
+    // k_census_bits: integer disparities whose coordinates x + dx + 0.5 - d are exact, tiles that fit, and lists dense enough
     bool whole = true;
     float lo = h_list[0], hi = h_list[0];
     for (int i = 0; i < D; ++i) {
@@ -278,7 +291,7 @@ int census_volume(const float *g1, const float *g2, int W, int H, int fs, const 
     }
     if (whole && W < 1048576 && hi - lo < 8192.0f) {
         const size_t sm = census_bits_smem(fs, D, (int)(hi - lo));
-        if (sm <= SMEM_MAX) {
+        if (sm <= SMEM_MAX && bits_pay(fs, D, (int)(hi - lo), sm)) {
             const int side = 2 * fs + 1, nw = (side * side - 1 + 31) / 32;
             auto kern = nw == 1   ? k_census_bits<1>
                         : nw == 2 ? k_census_bits<2>
@@ -289,7 +302,7 @@ int census_volume(const float *g1, const float *g2, int W, int H, int fs, const 
                                   : k_census_bits<0>;
             CNNCRF_CUDA(allow_smem(kern));
             {
-                CNNCRF_PROF("census", st);
+                CNNCRF_PROF("census_bits", st);
                 kern<<<dim3(ceil_div(W, CPX), H), CTH, sm, st>>>(g1, g2, W, H, fs, d_list, D, (int)lo, (int)hi, lambda, vol);
             }
             CNNCRF_CHECK_LAUNCH();
