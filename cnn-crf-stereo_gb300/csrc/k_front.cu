@@ -80,8 +80,12 @@ __device__ __forceinline__ double plane_sum(const double *rows, int Hp, int lane
 // same time); the warps are small and many, their loads eight pixels ahead.
 // Both sides of a KITTI pair in three launches take 72 us, in the ten launches
 // of one side at a time with the statistics in launches of their own 107 us.
+// TALL: more rows than ROW_CTAS CTAs per image (5 per SM) take once.  Each CTA of the second pass adds up all rows' sums for
+// the mean, which with a CTA per two rows grew with the square of the height: both passes of a 48 x 12000 pair 959 -> 203 us.
+// The others keep their kernel without the row loop (a KITTI pair 44 us, 49 with it).
 template <bool GRAY> __host__ __device__ constexpr int row_cta() { return GRAY ? 4 : 2; }
-template <bool GRAY, bool AL>
+constexpr int ROW_CTAS = 760;
+template <bool GRAY, bool AL, bool TALL>
 __global__ void __launch_bounds__(32 * row_cta<GRAY>() * (GRAY ? 1 : 3))
     k_rowsums(const float4 *__restrict__ ia, const float4 *__restrict__ ib, int n, int Wp, int Hp, int pass,
               double *__restrict__ rowsum)
@@ -89,7 +93,7 @@ __global__ void __launch_bounds__(32 * row_cta<GRAY>() * (GRAY ? 1 : 3))
     constexpr int NP = GRAY ? 1 : 3;
     __shared__ float smean[NP];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r = warp / NP, c = warp - r * NP, y = blockIdx.x * row_cta<GRAY>() + r;
+    const int r = warp / NP, c = warp - r * NP;
     double *rows = rowsum + (long)blockIdx.y * 6 * Hp;
     float mean = 0.0f;
     if (pass) {
@@ -101,17 +105,20 @@ __global__ void __launch_bounds__(32 * row_cta<GRAY>() * (GRAY ? 1 : 3))
         mean = smean[c];
         rows += 3 * Hp;
     }
-    if (y >= Hp) return;
-    const float4 *px = image(ia, ib, n, blockIdx.y, (long)Wp * Hp) + (long)y * Wp;
-    double s = 0.0;
+    const float4 *im = image(ia, ib, n, blockIdx.y, (long)Wp * Hp);
+    for (int y = blockIdx.x * row_cta<GRAY>() + r; y < Hp; y += gridDim.x * row_cta<GRAY>()) {
+        const float4 *px = im + (long)y * Wp;
+        double s = 0.0;
 #pragma unroll 8
-    for (int x = lane; x < Wp; x += 32) {
-        float v = plane_val<GRAY>(load_px<AL>(px + x), c);
-        if (pass) v = __fsub_rn(v, mean), v = __fmul_rn(v, v);
-        s += (double)v;
+        for (int x = lane; x < Wp; x += 32) {
+            float v = plane_val<GRAY>(load_px<AL>(px + x), c);
+            if (pass) v = __fsub_rn(v, mean), v = __fmul_rn(v, v);
+            s += (double)v;
+        }
+        s = warp_tree_sum(s);
+        if (lane == 0) rows[c * Hp + y] = s;
+        if (!TALL) return;
     }
-    s = warp_tree_sum(s);
-    if (lane == 0) rows[c * Hp + y] = s;
 }
 
 // (v - mean) / population std, and the coordinate planes.  A CTA takes the
@@ -156,7 +163,9 @@ int launch_normalize(const float4 *a, const float4 *b, int n, int nimg, int Wp, 
     const long npx = (long)Wp * Hp;
     for (int pass = 0; pass < 2; ++pass) {
         CNNCRF_PROF("rowsums", st);
-        k_rowsums<GRAY, AL><<<dim3(ceil_div(Hp, row_cta<GRAY>()), nimg), 32 * row_cta<GRAY>() * (GRAY ? 1 : 3), 0, st>>>(a, b, n, Wp, Hp, pass, rows);
+        const int ctas = std::min(ceil_div(Hp, row_cta<GRAY>()), ROW_CTAS);
+        const auto kern = ctas * row_cta<GRAY>() < Hp ? k_rowsums<GRAY, AL, true> : k_rowsums<GRAY, AL, false>;
+        kern<<<dim3(ctas, nimg), 32 * row_cta<GRAY>() * (GRAY ? 1 : 3), 0, st>>>(a, b, n, Wp, Hp, pass, rows);
     }
     {
         CNNCRF_PROF("norm_write", st);
