@@ -192,7 +192,7 @@ def crf_solve(cost, wx, wy, L1=1.0, L2=12.0, delta=2, total_it=4, shape=L.RHO_ST
 
 def crf_autotune(cost, wx, wy, L1=1.0, L2=12.0, delta=2, total_it=4, shape=L.RHO_STEP, slack=0.5, stream=None,
                  workspace=None):
-    """Measure every CRF tile on this single-pair problem and enter the fastest
+    """Measure the CRF tiles on this single-pair problem and enter the fastest
     in the tile table (cnncrf.tuning); synchronises."""
     H, W, D = cost.shape
     opt = crf_options(L1, L2, delta, total_it, shape, slack)

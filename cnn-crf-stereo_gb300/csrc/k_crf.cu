@@ -21,6 +21,8 @@
 // operations are exact (min) or single IEEE ops in the oracle's order, so the
 // labels equal the oracle's bit for bit.  Compiled with --fmad=false.
 #include <algorithm>
+#include <set>
+#include <tuple>
 #include <vector>
 
 #include "k_crf_chain.cuh"
@@ -285,8 +287,9 @@ int solve_impl(const float *cost, const float *wx, const float *wy, long wps, in
 }
 
 // time one H and one V pass of every candidate tile (events on `st`, best of
-// `reps`); the workspace's messages are overwritten, the next solve starts
-// afresh (its first H pass does not read them)
+// `reps`), tiles that run a pass as an earlier one does left out: between equal
+// launches only noise would choose.  The workspace's messages are overwritten,
+// the next solve starts afresh (its first H pass does not read them)
 int autotune_impl(const float *cost, const float *wx, const float *wy, long wps, int W, int H, int D, int np,
                   const CrfParams &p, void *ws, size_t ws_bytes, cudaStream_t st, CrfTile *best, float *ms_h,
                   float *ms_v, const void *costq, UnaryQ16 q)
@@ -304,9 +307,15 @@ int autotune_impl(const float *cost, const float *wx, const float *wy, long wps,
         cudaEvent_t e[3 * 3];
     };
     std::vector<Cand> cands;
+    std::set<std::tuple<bool, int, int>> forms[2]; // of the V and the H pass
+    auto is_new = [&](bool hpass, int ring, int wpb) {
+        if (!fits(D, hpass, wpb)) return false;
+        const CrfForm f = choose_form(a, hpass, ring, wpb);
+        return forms[hpass].insert({f.paired, f.buffers, f.paired ? 1 : f.wpb}).second;
+    };
     for (int r : rings)
         for (int b : wpbs) {
-            Cand c{r, b, fits(D, true, b), fits(D, false, b), {}};
+            Cand c{r, b, is_new(true, r, b), is_new(false, r, b), {}};
             if (c.h || c.v) cands.push_back(c);
         }
     int rc = CNNCRF_OK;

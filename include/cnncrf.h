@@ -263,10 +263,11 @@ int cnncrf_crf_solve_static(const float *d_cost, const float *d_wx, const float 
  * 8 nodes where shared memory then holds every chain of the launch, else two;
  * ring 4: two) and chains per CTA (1, 2 or 4) for the horizontal and the
  * vertical pass; passes with few chains (up to 8 per SM) run two warps per
- * chain, one chain per CTA, and three blocks at either depth.  Every tile gives the same labels and bound bit for bit; the fastest
- * depends on the label count, the chain lengths and the pairs per launch, so
- * the library keeps a process-wide table from (width, height, depth, npairs,
- * delta) to a tile.  Every solve (cnncrf_crf_solve, SlackProp, Stereo, the
+ * chain, one chain per CTA, and three blocks at either depth.  Every tile
+ * gives the same labels and bound bit for bit; the fastest depends on the
+ * label count, the chain lengths and the pairs per launch, so the library
+ * keeps a process-wide table from (width, height, depth, npairs, delta) to a
+ * tile.  Every solve (cnncrf_crf_solve, SlackProp, Stereo, the
  * batch) looks its shape up and runs the default tile (ring 8, 2 chains per
  * CTA, both passes) when the table has none.  The table is filled by the two
  * autotune calls below or set by hand, and can be saved to a text file and
@@ -288,9 +289,10 @@ int cnncrf_crf_tuning_count(int *n);
  * CNNCRF_EINVAL naming the line and changes nothing. */
 int cnncrf_crf_tuning_save(const char *path);
 int cnncrf_crf_tuning_load(const char *path);
-/* Measures every tile on this problem (one horizontal and one vertical pass
- * each, best of three, CUDA events on `stream`) and enters the fastest per
- * pass for (width, height, depth, 1, opt->delta).  Arguments as
+/* Measures the tiles on this problem (one horizontal and one vertical pass
+ * each, best of three, CUDA events on `stream`; of the tiles that run a pass
+ * the same way the first, the default before the others) and enters the
+ * fastest per pass for (width, height, depth, 1, opt->delta).  Arguments as
  * cnncrf_crf_solve; the workspace's contents are overwritten (the next solve
  * does not depend on them).  Synchronises the stream: not during a capture. */
 int cnncrf_crf_autotune(const float *d_cost, const float *d_wx, const float *d_wy, int width, int height,
