@@ -202,6 +202,7 @@ PROTOS = {
     "cnncrf_profile_query": ([C.c_char_p, C.POINTER(i32), C.POINTER(C.c_double)], i32),
     "cnncrf_profile_kernels": ([C.c_char_p, C.c_size_t], i32),
     "cnncrf_selftest_bounded_wait": ([i32, i32, vp], i32),
+    "cnncrf_selftest_tanh": ([C.c_uint32, C.c_uint64, C.POINTER(C.c_uint64), vp], i32),
 }
 
 _lib = None

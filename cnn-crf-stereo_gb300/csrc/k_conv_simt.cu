@@ -456,7 +456,7 @@ __device__ __forceinline__ unsigned long long vmul2(unsigned long long a, unsign
 //   2 |x| <= 18 needs no range case of expm1, 2^0 em1 + (2^0 - 1) is em1, and the quotient at |x| = 9 rounds to 1;
 //   the quotient E / (E + 2) by Markstein's correctly rounded division ("Computation of elementary functions on the
 //   IBM RISC System/6000 processor", 1990): a reciprocal y refined by one Newton step, q = E y, q + y (E - q (E + 2)).
-//   Its operands are those of the 2^27 or so floats between 2^-12 and 9, and each was compared with cnncrf_tanhf.
+//   Its operands are those of the 2^27 or so floats between 2^-12 and 9; selftest_tanh compares every float with cnncrf_tanhf.
 __device__ __forceinline__ float2 tanh_pair(float2 x)
 {
     auto both = [](float c) { return pack2(c, c); };
@@ -673,6 +673,24 @@ template <int CPW, int KP> int launch_patch(const ConvArgs &a, int Ho, int Wo, i
     return CNNCRF_OK;
 }
 
+// the floats of bit patterns first .. first + 2 npairs - 1 for which tanh_pair is not cnncrf_tanhf, counted (NaN equals NaN)
+__global__ void __launch_bounds__(256) k_tanh_sweep(uint32_t first, uint32_t npairs, unsigned long long *differing)
+{
+    uint32_t bad = 0;
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < npairs; i += (long)gridDim.x * blockDim.x) {
+        const uint32_t b = first + 2 * (uint32_t)i;
+        const float x[2] = {__uint_as_float(b), __uint_as_float(b + 1)};
+        const float2 t = tanh_pair(make_float2(x[0], x[1]));
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const float got = k ? t.y : t.x, want = cnncrf_tanhf(x[k]);
+            bad += __float_as_uint(got) != __float_as_uint(want) && !(got != got && want != want);
+        }
+    }
+    bad = __reduce_add_sync(0xffffffffu, bad);
+    if ((threadIdx.x & 31) == 0 && bad) atomicAdd(differing, (unsigned long long)bad);
+}
+
 __global__ void k_head2(const float *__restrict__ in, int npx, int Cin, const float *__restrict__ w,
                         float *__restrict__ out)
 {
@@ -771,6 +789,24 @@ int conv_simt(const ConvArgs &args, cudaStream_t st)
         else k_conv_simt<<<grid, 256, 0, st>>>(a, Ho, Wo, K);
     }
     CNNCRF_CHECK_LAUNCH();
+    return CNNCRF_OK;
+}
+
+int selftest_tanh(uint32_t first, uint64_t count, uint64_t *differing, cudaStream_t st)
+{
+    if (!differing || count < 2 || count % 2 || first + count > (1ull << 32))
+        return fail(CNNCRF_EINVAL, "selftest: floats %u .. + %llu", first, (unsigned long long)count);
+    DevBuf n;
+    CNNCRF_TRY(n.reserve(sizeof(unsigned long long)));
+    CNNCRF_CUDA(cudaMemsetAsync(n.get(), 0, sizeof(unsigned long long), st));
+    {
+        CNNCRF_PROF("tanh_sweep", st);
+        k_tanh_sweep<<<(int)std::min<uint64_t>((count / 2 + 255) / 256, 8 * 152), 256, 0, st>>>(first, (uint32_t)(count / 2),
+                                                                                            n.as<unsigned long long>());
+    }
+    CNNCRF_CHECK_LAUNCH();
+    CNNCRF_CUDA(cudaMemcpyAsync(differing, n.get(), sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
+    CNNCRF_CUDA(cudaStreamSynchronize(st));
     return CNNCRF_OK;
 }
 

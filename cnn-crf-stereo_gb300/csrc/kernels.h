@@ -297,6 +297,9 @@ int tv_iterate(float *u, float *u_, const float *u0, const float *qf, float *p, 
 // Bounded-wait self-test (k_selftest.cu): CNNCRF_ETIMEOUT when the probe's wait
 // on a barrier that nothing completes (arrive == 0) gave up after `polls` polls.
 int selftest_bounded_wait(int polls, int arrive, cudaStream_t st);
+// the floats of bit patterns first .. first + count - 1 whose tanh in the FP32 convolutions' epilogue (k_conv_simt.cu) is not
+// cnncrf_tanhf's, counted; count even
+int selftest_tanh(uint32_t first, uint64_t count, uint64_t *differing, cudaStream_t st);
 
 } // namespace k
 } // namespace cnncrf

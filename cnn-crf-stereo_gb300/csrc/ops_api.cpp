@@ -150,6 +150,12 @@ int cnncrf_selftest_bounded_wait(int polls, int arrive, cnncrf_stream_t stream)
     return k::selftest_bounded_wait(polls, arrive, (cudaStream_t)stream);
 }
 
+int cnncrf_selftest_tanh(uint32_t first, uint64_t count, uint64_t *differing, cnncrf_stream_t stream)
+{
+    clear_error();
+    return k::selftest_tanh(first, count, differing, (cudaStream_t)stream);
+}
+
 int cnncrf_crf_solve(const float *d_cost, const float *d_wx, const float *d_wy, int width, int height, int depth,
                      const cnncrf_crf_options *opt, int32_t *d_labels, double *lower_bound, void *d_workspace,
                      size_t workspace_bytes, cnncrf_stream_t stream)

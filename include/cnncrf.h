@@ -647,6 +647,12 @@ int cnncrf_profile_kernels(char *buf, size_t len);
  * probe moves no data and holds no tensor memory, so the context stays usable
  * after a timeout.  Synchronises the stream. */
 int cnncrf_selftest_bounded_wait(int polls, int arrive, cnncrf_stream_t stream);
+/* Self-test of the FP32 convolutions' packed tanh, whose equality with the
+ * library's scalar one (cnncrf_fmath.h) rests on this chip's reciprocal
+ * approximation: counts the floats of bit patterns first .. first + count - 1
+ * (count even, at most up to 2^32 - 1) on which the two differ; NaN equals
+ * NaN.  Synchronises the stream. */
+int cnncrf_selftest_tanh(uint32_t first, uint64_t count, uint64_t *differing, cnncrf_stream_t stream);
 
 #ifdef __cplusplus
 }
