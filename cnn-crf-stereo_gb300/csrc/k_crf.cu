@@ -147,10 +147,14 @@ size_t form_smem(int D, bool hpass, bool t16, int mode, const CrfForm &f)
 //   more chains the single warps hide each other's latency in less shared
 //   memory (1500 row chains: 604 us single, 624 us paired; 4968 column chains:
 //   481 and 526 us; 1242 column chains: 160 and 164 us), and so they do where
-//   the paired form's shared memory would not hold every chain at once.
+//   the paired form's shared memory would not hold every chain at once.  The
+//   forms cross at 8 to 11 chains per SM for 20 to 64 labels (128-node chains
+//   of 32 labels, H and V: 1064 of them 34 paired and 36 single, 36 and 36 us;
+//   1824 48 and 42, 50 and 42), at 6 to 7 for 75 and 128 (of 128 labels 912
+//   chains 46 and 51, 43 and 47; 1216 64 and 62, 54 and 51).
 //   Three block buffers where that leaves every chain of the launch resident,
-//   else two (KITTI pair's row chains: 258 us with three or four, 326 us with
-//   two; 1500 row chains, single: 604 us with two, 826 us with three).  A
+//   else two (KITTI pair's row chains: 258 us with three, 326 us with two;
+//   1500 row chains, single: 604 us with two, 826 us with three).  A
 //   tile's ring of 4 asks the single form for two.
 CrfForm choose_form(const CrfPassArgs &a, bool hpass, int ring, int wpb)
 {

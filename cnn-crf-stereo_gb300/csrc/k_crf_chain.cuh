@@ -32,7 +32,7 @@ struct CrfPassArgs {
     const float *wgt;   // wx (H pass) or wy (V pass), pair stride wps
     float *lbuf;        // each block's first forward message, [np][H][blocks][DP] in an H pass, [np][blocks][W][DP] in a V pass
     int W, H, D, np;
-    int DP;              // labels from one vector of phi and lbuf to the next: D rounded up to 4, or D (crf_pitch)
+    int DP;              // labels from one vector of phi and lbuf to the next: D rounded up to 4, or D (layout, k_crf.cu)
     long wps;
     Rho rp;
     int first;           // H pass of the first iteration: phi = 0, not read
@@ -44,7 +44,7 @@ struct CrfPassArgs {
 // how a pass runs: every choice gives the same bits
 struct CrfForm {
     bool paired; // two warps per chain, else one
-    int buffers; // blocks of BLK nodes in shared memory (2..4)
+    int buffers; // blocks of BLK nodes in shared memory (2 or 3)
     int wpb;     // chains per CTA (paired: always one)
 };
 
@@ -279,12 +279,11 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const void *src)
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-// all but the newest `left` groups (0..2) are complete
+// all but the newest `left` groups (0 or 1) are complete
 __device__ __forceinline__ void cp_wait_left(int left)
 {
     if (left == 0) cp_wait<0>();
-    else if (left == 1) cp_wait<1>();
-    else cp_wait<2>();
+    else cp_wait<1>();
 }
 
 // `cnt` consecutive vectors of 32 P labels of EB bytes that lie one after the
@@ -490,7 +489,7 @@ template <int P, bool ALIGNED> __device__ __forceinline__ void load_vec(const fl
 //   SPREAD      D not a multiple of 4: phi as above, the volume's vectors
 //               float by float into the same slots
 //   RAGGED      the 16-byte chunks that hold each vector, where the workspace
-//               does not hold phi at a pitch of whole chunks (crf_pitch)
+//               does not hold phi at a pitch of whole chunks (k_crf.cu)
 // Vectors at a pitch DP > D carry pad labels D..DP - 1 along.  The H pass
 // that starts a solve stores them as +inf, a V pass turns that into NaN, and
 // neither ever wins a minimum.  D = 75, of a 619 x 271 solve, against RAGGED
@@ -930,7 +929,7 @@ template <int P, int DELTA> int launch_dir(const CrfPassArgs &a, bool hpass, con
 template <int P> int launch_pass(const CrfPassArgs &a, bool hpass, int delta, const CrfForm &f, cudaStream_t st)
 {
     if (f.wpb < 1 || f.wpb > 4) return fail(CNNCRF_EINVAL, "crf: %d chains per CTA outside 1..4", f.wpb);
-    if (f.buffers < 2 || f.buffers > 4) return fail(CNNCRF_EINVAL, "crf: %d block buffers outside 2..4", f.buffers);
+    if (f.buffers < 2 || f.buffers > 3) return fail(CNNCRF_EINVAL, "crf: %d block buffers outside 2..3", f.buffers);
     // An offset whose rho reaches L2 never wins over the truncation: v_{k+-t} >= g, and adding the same w L2 rounds
     // monotonically, so v_{k+-t} + w rho_t >= g + w L2.  Those offsets are left out (the repository's truncated linear
     // term, L1 = 0.5, L2 = 1.5 at delta 3, computes two of its three), with the same bits
