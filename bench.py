@@ -567,12 +567,11 @@ def run_profile(args):
     return 0
 
 
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) measured with ncu on one-pair launches
-# of this workload, scaled to a launch of the 8-pair step (traffic grows with the images / chains):
-# k_conv_tc layer 3 over 2 images 449.9 MB; k_crf_chain H pass (reading the 16-bit unary) 904.7 MB and
-# V pass 630.6 MB per pair.
+# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) measured with ncu: k_conv_tc layer 3 over the 2 images of
+# one pair 449.9 MB, scaled by images; k_crf_chain H pass (reading the 16-bit unary) 7.98 GB and V pass 5.94 GB in
+# launches of 8 pairs (of one pair, whose second read partly hits the L2, 904 and 631 MB).
 CONV_TC_BYTES_PER_IMAGE = 449.9e6 / 2
-CRF_H_BYTES_PER_PAIR, CRF_V_BYTES_PER_PAIR = 904.7e6, 630.6e6
+CRF_H_BYTES_PER_PAIR, CRF_V_BYTES_PER_PAIR = 7.98e9 / 8, 5.94e9 / 8
 
 
 def make_batch(cnncrf, wl, B, precision, graph, stream, seed0, group_size=0):
@@ -981,8 +980,8 @@ def kitti_line(args, rank, world, local):
         tb = (CRF_H_BYTES_PER_PAIR + CRF_V_BYTES_PER_PAIR) / 2 * B
         crf_roof = {"kernel": "crf_h+crf_v", "bound": "hbm", "achieved": gbs, "peak": peaks["hbm_gbs"],
                     "unit": "GB/s", "frac": gbs / peaks["hbm_gbs"], "traffic": tb,
-                    "traffic_unit": "DRAM bytes per pass launch (%d pairs, mean of H and V; ncu, 1-pair launches "
-                                    "scaled); achieved counts the algorithmic 3 x N x D x 4 B per pass" % B,
+                    "traffic_unit": "DRAM bytes per pass launch (%d pairs, mean of H and V; ncu on launches of 8 "
+                                    "pairs, per pair); achieved counts the algorithmic 3 x N x D x 4 B per pass" % B,
                     "measured_gbs": tb * n / (t / 1000.0) / 1e9, "peak_source": peak_src}
 
     cpu = None

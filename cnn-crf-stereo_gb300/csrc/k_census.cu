@@ -87,8 +87,9 @@ __global__ void k_census(const float *__restrict__ g1, const float *__restrict__
 // filter size 7, and the (window^2 - 1)-entry table of lambda count / norm.
 // k_census compared all 225 positions per pixel and label, each with its own
 // two interpolation coordinates: 12.4 ms for 720 x 480 at 128 labels; this
-// takes 211 us, of which the population counts (16 per SM and cycle) are 67
-// and the volume's bytes 26.
+// takes 211 us.  Bound by issue (89 % of the cycles; 223 M warp instructions);
+// the population counts alone (16 per SM and cycle) are 67 us, the volume's
+// bytes 26.
 // NW: words per string, 0 for any.
 constexpr int CPX = 64, CTH = 256;
 

@@ -277,9 +277,11 @@ __global__ void __launch_bounds__(256)
 // Column px lies at px ^ 8 (c / 4 mod 4), which spreads the transposing stores
 // (8 pixels x 4 channel groups per warp) over the banks, and ^ 4 in every
 // other group of 32, which does the same for eight lanes' 16-byte loads.
-// Bound by the 24 floats a thread takes from shared memory per 64 fmas (24
-// wavefronts per warp and channel, 96 of an SM's cycles for 77 of its fmas)
-// and, under the softmax, the per-pixel epilogue.  A KITTI pair at D = 128, C
+// Bound by the latency of its phases: two CTAs per SM (shared memory), 8 warps,
+// load their whole tile, then compute, then gather and normalise, and issue in
+// 46 % of the cycles (FMA pipe 27 %, shared memory 38 % of its rate, DRAM 7 %).
+// A thread takes 24 floats from shared memory per 64 fmas: 24 wavefronts per
+// warp and channel, 96 of an SM's cycles for 77 of its fmas.  A KITTI pair at D = 128, C
 // = 100 with the softmax: 3.44 -> 1.04 ms; a 720 x 480 pair at D = 96 plus the
 // refinement's three labels 2.98 -> 0.81 ms; 256 x 192 at D = 32 0.214 ->
 // 0.066 ms (k_corr_band: scalar loads, 9 wavefronts per 20 fmas, its band's

@@ -514,8 +514,8 @@ template <int P, bool ALIGNED> __device__ __forceinline__ void load_vec(const fl
 //     once per block; one chain per CTA.
 //
 // What bounds it: many chains, DRAM (eight KITTI pairs at D = 128: the H pass
-// 7.9 GB in 1.18 ms, 6.7 TB/s, and the V pass 6.2 GB in 0.93 ms; with all
-// messages stored and read back 1.72 and 1.38 ms).  Few chains, the latency of
+// 7.98 GB by the counters in 1.22 ms, 6.56 TB/s, and the V pass 5.94 GB in 0.92
+// ms, 6.46 TB/s; with all messages stored and read back 1.72 and 1.38 ms).  Few chains, the latency of
 // a node's step, about 420 cycles for both sweeps of a KITTI pair's row: four
 // halo shuffles issue 4.3 cycles apart and return after 24, the warp minimum
 // after 18, and the copies of a block cost 18 cycles per instruction, which is
